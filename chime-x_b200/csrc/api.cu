@@ -93,6 +93,7 @@ cudaError_t build_tc_tables(chx_plan *p) {
     p->nunits = (int)units.size();
     p->grid = grid;
     p->tile_built = tile;
+    p->max_unit = tc_max_samples(units);
     p->has_split_units = false;
     for (const Unit &u : units) p->has_split_units |= (u.split != 0);
     return e;
@@ -121,6 +122,7 @@ int run_tc(chx_plan *p, const uint8_t *d_packed, int32_t *d_blocks, int map, int
     L.chans = (const ChanDesc *)p->d_chans;
     L.units = (const Unit *)p->d_units;
     L.nunits = p->nunits;
+    L.max_samples = p->max_unit;
     L.cta_offsets = (const int *)((const char *)p->d_units + (size_t)p->nunits * sizeof(Unit));
     L.out_base = (uint64_t)d_blocks;
     L.use_param_map = 1;

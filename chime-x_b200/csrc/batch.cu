@@ -67,7 +67,7 @@ bool tc_tune_lookup(int device, int E, int T, int *tile, int *split) {
 }  // namespace chx
 
 struct chx_batch {
-    int device = 0, ut = 1, n = 0, tile = 0, grid = 0, nunits = 0;
+    int device = 0, ut = 1, n = 0, tile = 0, grid = 0, nunits = 0, max_unit = 0;
     std::vector<chx_channel_desc> descs;
     chx::ChanDesc *d_chans = nullptr;
     void *d_units = nullptr;  // units then grid + 1 offsets
@@ -105,6 +105,7 @@ int record_batch(chx_batch *b, cudaStream_t st, int accumulate) {
     L.chans = b->d_chans;
     L.units = (const Unit *)b->d_units;
     L.nunits = b->nunits;
+    L.max_samples = b->max_unit;
     L.cta_offsets = (const int *)((const char *)b->d_units + (size_t)b->nunits * sizeof(Unit));
     L.out_base = 0;
     L.use_param_map = 0;
@@ -239,6 +240,7 @@ int chx_batch_create(chx_batch **out, int n, const chx_channel_desc *descs, int 
     std::vector<int> offsets;
     tc_schedule(units, b->grid, offsets);
     b->nunits = (int)units.size();
+    b->max_unit = tc_max_samples(units);
 
     const size_t ubytes = units.size() * sizeof(Unit);
     e = cudaMalloc(&b->d_chans, chans.size() * sizeof(ChanDesc));

@@ -49,6 +49,7 @@ struct chx_plan {
     int nunits;
     int grid;       // persistent CTAs (or CTA pairs) of a tensor-core launch
     int tile_built; // tile variant the tables were built for
+    int max_unit;   // samples of the longest unit
     bool has_split_units;  // some output cells receive several units (TMA reduce-add)
 };
 
@@ -154,6 +155,7 @@ struct TcLaunch {
     const ChanDesc *chans;  // device
     const Unit *units;      // device, grouped by CTA
     int nunits;
+    int max_samples;        // samples of the longest unit
     const int *cta_offsets; // device, grid + 1 entries
     uint64_t out_base;      // added to ChanDesc::out
     int use_param_map;      // 1: every channel uses the kernel-parameter map
@@ -174,6 +176,8 @@ void tc_schedule(std::vector<Unit> &u, int grid, std::vector<int> &offsets);
 // Makespan, in unit-cost units, of that assignment when every unit also pays
 // `handoff_stages` of its stages for the accumulator hand-off.
 long long tc_estimate_makespan(const std::vector<Unit> &u, int grid, int handoff_stages);
+// Samples of the longest unit.
+int tc_max_samples(const std::vector<Unit> &u);
 // Number of sample-range splits k (1-8) whose units, made by build(k, out),
 // have the shortest estimated makespan on the tile variant.
 int tc_choose_split(int tile, int sm_count,

@@ -318,6 +318,7 @@ extern "C" int chx_correlate_noalloc(const uint8_t *d_packed, int32_t *d_blocks,
     L.chans = reinterpret_cast<const ChanDesc *>(dscr + kOffChans);
     L.units = reinterpret_cast<const Unit *>(dscr + kOffUnits);
     L.nunits = P.n;
+    L.max_samples = std::min(T, kUnitMaxSamples);
     L.cta_offsets = reinterpret_cast<const int *>(dscr + kOffOffsets);
     L.out_base = (uint64_t)d_blocks;
     L.use_param_map = 1;

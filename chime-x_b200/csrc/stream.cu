@@ -488,6 +488,7 @@ int chx_stream_submit(chx_stream *s, int n, const int *ids, const uint8_t *const
     if (e == cudaSuccess && !units.empty()) {
         L.units = (const Unit *)sl.dev;
         L.nunits = (int)units.size();
+        L.max_samples = tc_max_samples(units);
         L.cta_offsets = (const int *)((const char *)sl.dev + ub);
         L.grid = grid;
         e = tc_pair_launch(L, nullptr, nullptr, st);
@@ -495,6 +496,7 @@ int chx_stream_submit(chx_stream *s, int n, const int *ids, const uint8_t *const
     if (e == cudaSuccess && !units1.empty()) {
         L.units = (const Unit *)((const char *)sl.dev + u1b0);
         L.nunits = (int)units1.size();
+        L.max_samples = tc_max_samples(units1);
         L.cta_offsets = (const int *)((const char *)sl.dev + u1b0 + u1b);
         L.grid = grid1;
         e = tc_launch(L, nullptr, nullptr, st);

@@ -1,6 +1,6 @@
 // tc_cluster.cuh -- helpers of the SM-pair (cta_group::2) tensor-core
-// kernels: cluster rank and barrier, remote mbarrier arrivals, cluster-scope
-// bounded waits, and the pair MMA and its multicast commit.
+// kernels: cluster rank and barrier, remote mbarrier arrivals, and the
+// pair MMAs of one stage and their multicast commit.
 #pragma once
 
 #include "tc_common.cuh"
@@ -26,47 +26,45 @@ __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
+// One lane of a converged warp (the same one each time).
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t p;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
+        : "=r"(p));
+    return p;
 }
-// Bounded wait with cluster-scope acquire (barriers that receive arrivals
-// from the other CTA of the pair).
-static __device__ __noinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
-                                               volatile int *abort_flag) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    const uint64_t t0 = globaltimer();
-    while (true) {
-#pragma unroll 1
-        for (int i = 0; i < 64; i++)
-            if (mbar_try_wait_cluster(bar, parity)) return true;
-        if (*abort_flag) return false;
-        if (globaltimer() - t0 > kWaitLimitNs) return false;
-    }
-}
-__device__ __forceinline__ void mma_i8_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                            uint32_t idesc, uint32_t accumulate) {
+
+// The four MMAs of one stage, issued by the lane with lead = 1 of a converged
+// warp.  acc = 0 starts new sums.  Re and Im MMAs alternate, so that an MMA does not wait
+// for the previous one's update of its accumulator.
+//   Re (d0) = R X + I Y,   Im (d1) = I X + N Y
+__device__ __forceinline__ void mma_stage_pair(uint32_t lead, uint32_t d0, uint32_t d1, uint64_t r,
+                                               uint64_t i, uint64_t n, uint64_t x, uint64_t y,
+                                               uint32_t idesc, uint32_t acc) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p, q, t;\n\t"
+        "setp.ne.b32 q, %0, 0;\n\t"
+        "setp.ne.b32 p, %9, 0;\n\t"
+        "setp.eq.b32 t, 0, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::i8 [%1], %3, %6, %8, p;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::i8 [%2], %4, %6, %8, p;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::i8 [%1], %4, %7, %8, t;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::i8 [%2], %5, %7, %8, t;\n\t}" ::"r"(lead),
+        "r"(d0), "r"(d1), "l"(r), "l"(i), "l"(n), "l"(x), "l"(y), "r"(idesc), "r"(acc)
         : "memory");
 }
-// Commit of the pair's MMAs, arriving on the barrier at `bar` in both CTAs.
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
+// Commit of the lead lane's MMAs, arriving on the barrier at `bar` in both CTAs.
+__device__ __forceinline__ void mma_commit_pair(uint32_t lead, uint32_t bar) {
     const uint16_t mask = 0x3;
     asm volatile(
-        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
-        " [%0], %1;" ::"r"(bar),
-        "h"(mask)
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %2, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster"
+        ".multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar),
+        "h"(mask), "r"(lead)
         : "memory");
 }
 

@@ -56,6 +56,42 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
     if (mbar_try_wait(bar, parity)) return true;
     return mbar_wait_slow(bar, parity, abort_flag);
 }
+// try_wait with cluster-scope acquire (barriers with arrivals from the other
+// CTA of a pair).
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// Bounded wait of a converged warp: every lane waits and all get the same
+// answer, so that the warp stays converged whatever happens.
+template <bool CLUSTER>
+static __device__ __noinline__ bool mbar_wait_warp_slow(uint32_t bar, uint32_t parity,
+                                                        volatile int *abort_flag) {
+    const uint64_t t0 = globaltimer();
+    while (true) {
+#pragma unroll 1
+        for (int i = 0; i < 64; i++) {
+            const bool done = CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity);
+            if (__all_sync(0xffffffffu, done)) return true;
+        }
+        if (__any_sync(0xffffffffu, *abort_flag != 0 || globaltimer() - t0 > kWaitLimitNs))
+            return false;
+    }
+}
+template <bool CLUSTER = false>
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity,
+                                               volatile int *abort_flag) {
+    const bool done = CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity);
+    if (__all_sync(0xffffffffu, done)) return true;
+    return mbar_wait_warp_slow<CLUSTER>(bar, parity, abort_flag);
+}
 // Bounded wait ignoring the abort flag (draining in-flight asynchronous work).
 static __device__ __noinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parity) {
     const uint64_t t0 = globaltimer();
@@ -217,6 +253,35 @@ __device__ __forceinline__ void xconv(uint32_t w, uint32_t &xr, uint32_t &xi) {
     } else {
         xr = w & 0xF0F0F0F0u;
         xi = (w << 4) & 0xF0F0F0F0u;
+    }
+}
+
+// The SM-pair kernel's y rows, scaled by 2^a (a = 0 or 3, fixed per launch):
+// R = yr 2^a, I = yi 2^a, N = -yr 2^a (and the offset-domain maps alike);
+// tc_pair_correlator.cu says why.
+struct YScale {
+    uint32_t shr, shl, mask, add, sub;  // nibble shifts, nibble mask, offsets of +/- rows
+    __device__ __forceinline__ explicit YScale(uint32_t a)
+        : shr(4 - a), shl(a), mask(0x0F0F0F0Fu << a), add(0x01010101u * (128u - (8u << a))),
+          sub(0x01010101u * (128u + (8u << a))) {}
+};
+template <int MAP>
+__device__ __forceinline__ void yconv_scaled(const YScale &c, uint32_t w, uint32_t &r, uint32_t &i,
+                                             uint32_t &n) {
+    const uint32_t hi = (w >> c.shr) & c.mask;
+    const uint32_t lo = (w << c.shl) & c.mask;
+    if (MAP == MAP_EXACT) {  // yr, yi, -yr
+        r = (hi + c.add) ^ 0x80808080u;
+        i = (lo + c.add) ^ 0x80808080u;
+        n = (c.sub - hi) ^ 0x80808080u;
+    } else if (MAP == MAP_CONF) {  // y'r, y'i, -y'r
+        r = hi;
+        i = lo;
+        n = neg(hi);
+    } else {  // y'r, -(15 - y'i), -y'r
+        r = hi;
+        i = neg(lo ^ c.mask);
+        n = neg(hi);
     }
 }
 

@@ -578,6 +578,12 @@ void tc_schedule(std::vector<Unit> &u, int grid, std::vector<int> &offsets) {
     u.swap(out);
 }
 
+int tc_max_samples(const std::vector<Unit> &u) {
+    int m = 0;
+    for (const Unit &x : u) m = std::max(m, x.t1 - x.t0);
+    return m;
+}
+
 long long tc_estimate_makespan(const std::vector<Unit> &u, int grid, int handoff_stages) {
     if (grid < 1) grid = 1;
     std::vector<long long> cost(u.size());

@@ -10,22 +10,44 @@
 // third, for the same tensor work per SM as the 1-SM kernel.  Each CTA's TMEM
 // receives its 128 rows x 256 columns of Re (columns 0-255) and Im (256-511).
 //
-// Operand formulation, layout, value maps and the stage-pair MMA order are the
-// 1-SM kernel's (tc_correlator.cu); per CTA a 32-sample stage holds y
-// [R0 R1 R2 R3 | I0 I1 I2 I3 | N0 N1 N2 N3] (12 KiB) and x
-// [X0 X1 X2 X3 | Y0 Y1 Y2 Y3] (8 KiB), each part an 8-sample atom.
+// Operand formulation and layout are the 1-SM kernel's (tc_correlator.cu); per
+// CTA a 32-sample stage holds y [R0 R1 R2 R3 | I0 I1 I2 I3 | N0 N1 N2 N3]
+// (12 KiB) and x [X0 X1 X2 X3 | Y0 Y1 Y2 Y3] (8 KiB), each part an 8-sample atom.
 //
-// Warps: 0-15 unpack (0-7 y, 8-15 x), 16 TMA producer, 17 MMA issuer (CTA 0),
-// 18-25 epilogue.  The epilogue warps drain the accumulators of one unit while
-// the unpack warps convert the next; each 32 x 32-word output tile goes from
-// TMEM through a swizzled staging tile in shared memory to a TMA store (or
-// reduce-add) into the block buffer.
+// Warps: 0-15 unpack, 16 TMA producer, 17 MMA issuer (CTA 0), 18-25 epilogue.
+// The epilogue warps drain the accumulators of one unit while the unpack warps
+// convert the next; each 32 x 32-word output tile goes from TMEM through a
+// swizzled staging tile in shared memory to a TMA store (or reduce-add) into
+// the block buffer.
+//
+// What bounds the main loop: the tensor pipe.  A stage takes 510 cycles
+// (clock64 around the MMA loop) of the 512 that its four M256 N256 K32 MMAs
+// need; under a long load the power cap lowers the clock below 1965 MHz and
+// that, not the pipeline, sets the time.  Three things got it there from 740-770
+// cycles (E = 2048, F = 8, T = 16384):
+//   * The unpack warps work in kGroups groups, stage s in group s % kGroups, so
+//     that four stages are in different phases (load, convert, store, fence) at
+//     a time.  All 16 warps on one stage moved through the phases in step and
+//     took 676 cycles a stage even without any MMA.
+//   * The MMA warp stays converged and issues with an elected lane's predicate.
+//     Issued from a lane == 0 branch, the MMAs and the waits between them queued
+//     up one behind the other and left the tensor pipe idle for about 300 cycles
+//     at every commit (670 cycles a stage).
+//   * The packed ring has 8 stages (see kPkStages).
+//
+// Why the y rows are scaled (YScale).  Under the power cap the toggling of the
+// operand bits sets the clock: x = 16 xr instead of xr (no sign extension in the
+// low nibble's place) is worth 7 % of the time of a sustained load, y = 8 yr
+// instead of yr another 3 % (687 vs 710 us).  8 is the largest factor that
+// leaves -y in int8; |acc| <= 8 * 16 * 128 T then fits int32 for T < 2^17 (the
+// offset-domain maps: 8 * 16 * 450 T, T <= 37282), so launches whose longest
+// unit exceeds kScaledMaxSamples keep y unscaled.
 //
 // Synchronisation across the pair:
-//   full_pair[p] in CTA 0; every unpack warp of both CTAs arrives once per
-//                stage pair (one lane, after its lanes' proxy fences) -> the
-//                MMA thread waits.
-//   empty_pair   in both CTAs; CTA 0's commit arrives on both (multicast).
+//   full_op[s]   in CTA 0; the kGroupWarps unpack warps of the stage's group
+//                arrive in both CTAs (one lane each, after its lanes' proxy
+//                fences) -> the MMA warp waits.
+//   empty_op[s]  in both CTAs; CTA 0's commit arrives on both (multicast).
 //   acc_full     in both CTAs; CTA 0's commit arrives on both (multicast).
 //   acc_empty    in CTA 0; every epilogue warp of both CTAs arrives.
 // TMA loads, the packed ring and its barriers are local to each CTA.  Both
@@ -45,18 +67,27 @@ namespace {
 using namespace tc;
 
 constexpr int kStageSamples = kUnitStageSamples;
-constexpr int kOpSlots = 4;     // 2 stage pairs
-constexpr int kPairs = kOpSlots / 2;
-constexpr int kPkStages = 4;
+constexpr int kOpSlots = 4;     // operand slots, one stage each
+constexpr int kUnpackWarps = 16;
+constexpr int kGroups = 4;      // unpack groups: stage s belongs to group s % kGroups
+constexpr int kGroupWarps = kUnpackWarps / kGroups;
+// Packed stages.  A group may run ahead of another group's late TMA load, and
+// the parity wait on a packed slot must not mistake its previous phase for the
+// wanted one.  Before stage s a group has finished stage s - kGroups, whose
+// operand slot was free only once the MMAs had consumed stage
+// s - kGroups - kOpSlots: with kPkStages >= kGroups + kOpSlots that includes
+// the slot's previous stage.
+constexpr int kPkStages = 8;
+static_assert(kPkStages >= kGroups + kOpSlots, "parity of the packed ring");
+constexpr int kScaledMaxSamples = 1 << 15;  // longest unit with y scaled by 8
 constexpr int kYOpBytes = 12 * 1024;
 constexpr int kXOpBytes = 8 * 1024;
 constexpr int kPkBytes = kStageSamples * 128;  // one 128-element tile, 4 KiB
-constexpr int kUnpackWarps = 16;
 constexpr int kProducerWarp = 16;
 constexpr int kMmaWarp = 17;
 constexpr int kEpiWarp0 = 18;   // epilogue warps from here on, lane quarter = warp % 4
 constexpr int kEpiWarps = 8;    // 4 or 8: each warp drains 8 / (kEpiWarps / 4) column blocks
-constexpr int kEpiTiles = 3;    // 4 KiB output staging tiles per epilogue warp
+constexpr int kEpiTiles = 2;    // 4 KiB output staging tiles per epilogue warp
 constexpr int kEpiStageBytes = kEpiTiles * 4096;
 constexpr int kEpiBlocks = 8 / (kEpiWarps / 4);
 constexpr int kThreads = (kEpiWarp0 + kEpiWarps) * 32;
@@ -75,9 +106,9 @@ static_assert(kSmemBytes <= 232448, "shared memory per CTA");
 // Barrier offsets inside the barrier block (8 bytes each).
 constexpr int kBarFullPk = 0;
 constexpr int kBarEmptyPk = kBarFullPk + kPkStages;
-constexpr int kBarFullPair = kBarEmptyPk + kPkStages;
-constexpr int kBarEmptyPair = kBarFullPair + kPairs;
-constexpr int kBarAccFull = kBarEmptyPair + kPairs;
+constexpr int kBarFullOp = kBarEmptyPk + kPkStages;
+constexpr int kBarEmptyOp = kBarFullOp + kOpSlots;
+constexpr int kBarAccFull = kBarEmptyOp + kOpSlots;
 constexpr int kBarAccEmpty = kBarAccFull + 1;
 constexpr int kBarDrain = kBarAccEmpty + 1;
 constexpr int kBarCount = kBarDrain + 1;
@@ -91,6 +122,7 @@ struct KParams {
     int use_param_map;
     int ut;
     int accumulate;
+    uint32_t yscale;  // y rows are scaled by 2^yscale
     int *err;
 };
 
@@ -110,17 +142,20 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
         reinterpret_cast<volatile uint32_t *>(smem + kOffBars + 8 * kBarCount);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // warp-uniform
+    const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const int cluster = blockIdx.x >> 1;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kPkStages; s++) {
             mbar_init(bar(kBarFullPk + s), 1);
-            mbar_init(bar(kBarEmptyPk + s), kUnpackWarps);
+            mbar_init(bar(kBarEmptyPk + s), kGroupWarps);
         }
-        for (int s = 0; s < kPairs; s++) mbar_init(bar(kBarFullPair + s), 2 * kUnpackWarps);
-        for (int s = 0; s < kPairs; s++) mbar_init(bar(kBarEmptyPair + s), 1);
+        for (int s = 0; s < kOpSlots; s++) {
+            mbar_init(bar(kBarFullOp + s), 2 * kGroupWarps);
+            mbar_init(bar(kBarEmptyOp + s), 1);
+        }
         mbar_init(bar(kBarAccFull), 1);
         mbar_init(bar(kBarAccEmpty), 2 * kEpiWarps);
         mbar_init(bar(kBarDrain), 1);
@@ -156,7 +191,7 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
                 const int tx = 2 * ((U.tyx >> 10) & 1023) + (int)rank;
                 const int nst = (U.t1 - U.t0 + kStageSamples - 1) / kStageSamples;
                 for (int it = 0; it < nst; it++, g++) {
-                    const int s = g % kPkStages;
+                    const uint32_t s = g % kPkStages;
                     const uint32_t ph = (g / kPkStages) & 1;
                     if (!mbar_wait(bar(kBarEmptyPk + s), ph ^ 1, abort_flag)) {
                         ok = false;
@@ -180,165 +215,137 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
         __syncwarp();
     } else if (warp == kMmaWarp) {
         // ------------------------------------------------- MMA issuer (CTA 0 only)
-        if (lane == 0) {
-            if (rank == 0) {
-                uint32_t gp = 0, acc_phase = 0;
-                bool ok = true;
-                const bool b_signed = (MAP == MAP_EXACT);
-                // M = 256 over the pair, N = 256 over the pair.
-                const uint32_t idesc = (2u << 4) | (1u << 7) | ((b_signed ? 1u : 0u) << 10) |
-                                       (1u << 15) | (1u << 16) | ((256u >> 3) << 17) |
-                                       ((256u >> 4) << 24);
-                // per stage: y rows R, I, N and x rows X, Y, 32 samples each
-                const uint64_t dR = sdesc(op_y, 1024, 1024);
-                const uint64_t dI = sdesc(op_y + 4096, 1024, 1024);
-                const uint64_t dN = sdesc(op_y + 8192, 1024, 1024);
-                const uint64_t dX = sdesc(op_x, 1024, 1024), dY = sdesc(op_x + 4096, 1024, 1024);
-                for (int u = first; u < last && ok; u++) {
-                    const Unit U = P.units[u];
-                    const int nst = (U.t1 - U.t0 + kStageSamples - 1) / kStageSamples;
-                    const int npair = (nst + 1) / 2;
-                    if (!mbar_wait_cluster(bar(kBarAccEmpty), acc_phase ^ 1, abort_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    for (int ip = 0; ip < npair; ip++, gp++) {
-                        const int ps = (int)(gp % kPairs);
-                        const uint32_t ph = (gp / kPairs) & 1;
-                        const int nin = (2 * ip + 1 < nst) ? 2 : 1;
-                        if (!mbar_wait_cluster(bar(kBarFullPair + ps), ph, abort_flag)) {
-                            ok = false;
-                            break;
-                        }
-                        tc_fence_after();
-                        const uint32_t acc = (ip > 0) ? 1u : 0u;
-                        // Re and Im MMAs alternate: consecutive MMAs then go
-                        // to different accumulators and need not wait for
-                        // each other's TMEM update (8-9 % faster than four
-                        // Re MMAs followed by four Im MMAs).
-                        for (int j = 0; j < nin; j++) {
-                            const int s = 2 * ps + j;
-                            const uint64_t so_y = (uint64_t)((s * kYOpBytes) >> 4);
-                            const uint64_t so_x = (uint64_t)((s * kXOpBytes) >> 4);
-                            const uint32_t a0 = (j > 0) ? 1u : acc;
-                            mma_i8_pair(tmem_base, dR + so_y, dX + so_x, idesc, a0);        // Re += R X
-                            mma_i8_pair(tmem_base + 256, dI + so_y, dX + so_x, idesc, a0);  // Im += I X
-                            mma_i8_pair(tmem_base, dI + so_y, dY + so_x, idesc, 1u);        // Re += I Y
-                            mma_i8_pair(tmem_base + 256, dN + so_y, dY + so_x, idesc, 1u);  // Im += N Y
-                        }
-                        mma_commit_pair(bar(kBarEmptyPair + ps));
-                    }
+        // The whole warp runs the loop; the elected lane issues.
+        if (rank == 0) {
+            const uint32_t lead = elect_one();
+            // M = 256 over the pair, N = 256 over the pair; x unsigned in the
+            // offset-domain maps, y always signed.
+            const uint32_t idesc = (2u << 4) | (1u << 7) | ((MAP == MAP_EXACT ? 1u : 0u) << 10) |
+                                   (1u << 15) | (1u << 16) | ((256u >> 3) << 17) |
+                                   ((256u >> 4) << 24);
+            // per stage: y rows R, I, N and x rows X, Y, 32 samples each
+            const uint64_t dR = sdesc(op_y, 1024, 1024);
+            const uint64_t dI = sdesc(op_y + 4096, 1024, 1024);
+            const uint64_t dN = sdesc(op_y + 8192, 1024, 1024);
+            const uint64_t dX = sdesc(op_x, 1024, 1024), dY = sdesc(op_x + 4096, 1024, 1024);
+            uint32_t s = 0, ph = 0, acc_phase = 0;  // operand slot, its phase
+            bool ok = true;
+            for (int u = first; u < last && ok; u++) {
+                const int t0 = P.units[u].t0, t1 = P.units[u].t1;
+                const int nst = (t1 - t0 + kStageSamples - 1) / kStageSamples;
+                ok = mbar_wait_warp<true>(bar(kBarAccEmpty), acc_phase ^ 1, abort_flag);
+                if (!ok) break;
+                tc_fence_after();
+                for (int it = 0; it < nst; it++) {
+                    ok = mbar_wait_warp<true>(bar(kBarFullOp) + 8 * s, ph, abort_flag);
                     if (!ok) break;
-                    mma_commit_pair(bar(kBarAccFull));
-                    acc_phase ^= 1;
+                    tc_fence_after();
+                    const uint32_t so_y = s * (kYOpBytes >> 4), so_x = s * (kXOpBytes >> 4);
+                    mma_stage_pair(lead, tmem_base, tmem_base + 256, dR + so_y, dI + so_y, dN + so_y,
+                                   dX + so_x, dY + so_x, idesc, it > 0 ? 1u : 0u);
+                    mma_commit_pair(lead, bar(kBarEmptyOp) + 8 * s);
+                    s = s + 1 == kOpSlots ? 0 : s + 1;
+                    ph ^= s == 0 ? 1u : 0u;
                 }
-                if (!ok) {
-                    atomicOr(P.err, 0x200);
-                    *abort_flag = 1;
-                    asm volatile(
-                        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64"
-                        " [%0];" ::"r"(bar(kBarDrain))
-                        : "memory");
-                    mbar_wait_drain(bar(kBarDrain), 0);
-                }
+                if (!ok) break;
+                mma_commit_pair(lead, bar(kBarAccFull));
+                acc_phase ^= 1;
+            }
+            if (!ok && lead) {
+                atomicOr(P.err, 0x200);
+                *abort_flag = 1;
+                asm volatile(
+                    "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64"
+                    " [%0];" ::"r"(bar(kBarDrain))
+                    : "memory");
+                mbar_wait_drain(bar(kBarDrain), 0);
             }
         }
         __syncwarp();
     } else if (warp < kUnpackWarps) {
         // ------------------------------------------------- unpack (both CTAs)
-        const int tid = threadIdx.x;  // 0..511
-        const bool is_y = tid < 256;
-        const int c = tid & 255;
-        const int sy = c >> 3, gy = c & 7;
-        const uint32_t ry = (uint32_t)(sy & 7), by8 = (uint32_t)(sy >> 3);
-        const uint32_t ldoff = (uint32_t)(sy * 128 + gy * 16);
-        const uint32_t st_a = by8 * 1024 + swz(ry, gy);  // R or X; I / Y at +4K, N at +8K
-        const uint32_t full_pair_leader = mapa(bar(kBarFullPair), 0);
-        uint32_t g = 0, gp = 0;
+        // Warp gw of a group converts samples 8 gw .. 8 gw + 7 (one atom) of the
+        // stage's y and x tiles: each lane two 16-byte chunks of each tile,
+        // chunk lane & 7 of the samples lane >> 3 and (lane >> 3) + 4.
+        const int grp = warp / kGroupWarps, gw = warp % kGroupWarps;
+        const int r0 = lane >> 3;
+        const uint32_t ldoff = (uint32_t)(gw * 1024 + lane * 16);
+        const uint32_t st0 = (uint32_t)gw * 1024 + swz(r0, lane & 7);
+        const uint32_t st1 = (uint32_t)gw * 1024 + swz(r0 + 4, lane & 7);
+        const uint32_t full_op_leader = mapa(bar(kBarFullOp), 0);
+        const YScale ys(P.yscale);
+        uint32_t g = 0;  // stages of the units before this one
         bool ok = true;
         for (int u = first; u < last && ok; u++) {
-            const Unit U = P.units[u];
-            const int nst = (U.t1 - U.t0 + kStageSamples - 1) / kStageSamples;
-            // Stages are unpacked two at a time (one stage pair): both loads
-            // and conversions first, then one wait for the operand slots, the
-            // stores of both stages, one proxy fence and one arrive per warp.
-            for (int it = 0; it < nst; it += 2, gp++) {
-                const int nin = (it + 1 < nst) ? 2 : 1;
-                uint32_t v0[2][4], v1[2][4], v2[2][4];
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    if (j >= nin) break;
-                    const uint32_t gs = g + (uint32_t)j;
-                    const int ps = (int)(gs % kPkStages);
-                    if (!mbar_wait(bar(kBarFullPk + ps), (gs / kPkStages) & 1, abort_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    const bool valid = (U.t0 + (it + j) * kStageSamples + sy) < U.t1;
-                    if (is_y) {
-                        const uint4 w = lds128(pk_y + ps * kPkBytes + ldoff);
-                        yconv<MAP>(w.x, v0[j][0], v1[j][0], v2[j][0]);
-                        yconv<MAP>(w.y, v0[j][1], v1[j][1], v2[j][1]);
-                        yconv<MAP>(w.z, v0[j][2], v1[j][2], v2[j][2]);
-                        yconv<MAP>(w.w, v0[j][3], v1[j][3], v2[j][3]);
-                    } else {
-                        const uint4 w = lds128(pk_x + ps * kPkBytes + ldoff);
-                        xconv<MAP>(w.x, v0[j][0], v1[j][0]);
-                        xconv<MAP>(w.y, v0[j][1], v1[j][1]);
-                        xconv<MAP>(w.z, v0[j][2], v1[j][2]);
-                        xconv<MAP>(w.w, v0[j][3], v1[j][3]);
-#pragma unroll
-                        for (int k = 0; k < 4; k++) v2[j][k] = 0u;
-                    }
-                    if (!valid) {
-#pragma unroll
-                        for (int k = 0; k < 4; k++) v0[j][k] = v1[j][k] = v2[j][k] = 0u;
-                    }
-                    // The converted registers depend on the loads, and
-                    // __syncwarp orders every lane before lane 0's arrive:
-                    // one arrival per warp frees the slot.
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar(kBarEmptyPk + ps));
-                }
+            const int t0 = P.units[u].t0, t1 = P.units[u].t1;
+            const int nst = (t1 - t0 + kStageSamples - 1) / kStageSamples;
+            for (int it = (int)(((uint32_t)grp - g) % kGroups); it < nst; it += kGroups) {
+                const uint32_t gs = g + (uint32_t)it;
+                const uint32_t ps = gs % kPkStages;
+                ok = mbar_wait_warp(bar(kBarFullPk) + 8 * ps, (gs / kPkStages) & 1, abort_flag);
                 if (!ok) break;
-                g += (uint32_t)nin;
-
-                const int pslot = (int)(gp % kPairs);
-                if (!mbar_wait(bar(kBarEmptyPair + pslot), ((gp / kPairs) & 1) ^ 1, abort_flag)) {
-                    ok = false;
-                    break;
-                }
+                uint4 wy[2], wx[2];
+                wy[0] = lds128(pk_y + ps * kPkBytes + ldoff);
+                wy[1] = lds128(pk_y + ps * kPkBytes + ldoff + 512);
+                wx[0] = lds128(pk_x + ps * kPkBytes + ldoff);
+                wx[1] = lds128(pk_x + ps * kPkBytes + ldoff + 512);
+                uint32_t y[2][3][4], x[2][2][4];  // [chunk][row R I N / X Y][word]
 #pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    if (j >= nin) break;
-                    const int os = 2 * pslot + j;
-                    if (is_y) {
-                        const uint32_t ya = op_y + os * kYOpBytes + st_a;
-                        sts128(ya, v0[j][0], v0[j][1], v0[j][2], v0[j][3]);                // R
-                        sts128(ya + 4096, v1[j][0], v1[j][1], v1[j][2], v1[j][3]);  // I
-                        sts128(ya + 8192, v2[j][0], v2[j][1], v2[j][2], v2[j][3]);  // N
-                    } else {
-                        const uint32_t xa = op_x + os * kXOpBytes + st_a;
-                        sts128(xa, v0[j][0], v0[j][1], v0[j][2], v0[j][3]);         // X
-                        sts128(xa + 4096, v1[j][0], v1[j][1], v1[j][2], v1[j][3]);  // Y
+                for (int k = 0; k < 2; k++) {
+                    const uint32_t a[4] = {wy[k].x, wy[k].y, wy[k].z, wy[k].w};
+                    const uint32_t b[4] = {wx[k].x, wx[k].y, wx[k].z, wx[k].w};
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        yconv_scaled<MAP>(ys, a[q], y[k][0][q], y[k][1][q], y[k][2][q]);
+                        xconv<MAP>(b[q], x[k][0][q], x[k][1][q]);
                     }
+                }
+                // The converted registers depend on the loads, and __syncwarp
+                // orders every lane before lane 0's arrive: one arrival per
+                // warp frees the slot.
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar(kBarEmptyPk) + 8 * ps);
+                if (t0 + (it + 1) * kStageSamples > t1) {  // samples past the unit are zero
+#pragma unroll
+                    for (int k = 0; k < 2; k++)
+                        if (t0 + it * kStageSamples + 8 * gw + r0 + 4 * k >= t1) {
+#pragma unroll
+                            for (int q = 0; q < 4; q++) {
+                                y[k][0][q] = y[k][1][q] = y[k][2][q] = 0u;
+                                x[k][0][q] = x[k][1][q] = 0u;
+                            }
+                        }
+                }
+                const uint32_t os = gs % kOpSlots;
+                ok = mbar_wait_warp(bar(kBarEmptyOp) + 8 * os, ((gs / kOpSlots) & 1) ^ 1, abort_flag);
+                if (!ok) break;
+                const uint32_t ya = op_y + os * kYOpBytes, xa = op_x + os * kXOpBytes;
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const uint32_t st = k ? st1 : st0;
+#pragma unroll
+                    for (int r = 0; r < 3; r++)
+                        sts128(ya + r * 4096 + st, y[k][r][0], y[k][r][1], y[k][r][2], y[k][r][3]);
+#pragma unroll
+                    for (int r = 0; r < 2; r++)
+                        sts128(xa + r * 4096 + st, x[k][r][0], x[k][r][1], x[k][r][2], x[k][r][3]);
                 }
                 fence_proxy_async();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(full_pair_leader + 8 * pslot);
+                if (lane == 0) mbar_arrive_cluster(full_op_leader + 8 * os);
             }
+            g += (uint32_t)nst;
         }
-        if (!ok) {
+        if (!ok && lane == 0) {
             atomicOr(P.err, 0x400);
             *abort_flag = 1;
         }
-        // No multicast arrival may still be on its way to this CTA's pair
+        // No multicast arrival may still be on its way to this CTA's operand
         // barriers when it retires: thread 0 waits for the last phase of each.
-        if (tid == 0)
-            for (int k = 0; k < kPairs; k++)
-                if (gp > (uint32_t)k)  // pairs gp' < gp with slot k: their last phase
-                    mbar_wait_drain(bar(kBarEmptyPair + k), ((gp - 1 - k) / kPairs) & 1);
+        if (threadIdx.x == 0)
+            for (uint32_t k = 0; k < kOpSlots; k++)
+                if (g > k)  // stages < g in slot k: their last phase
+                    mbar_wait_drain(bar(kBarEmptyOp) + 8 * k, ((g - 1 - k) / kOpSlots) & 1);
     } else {
         // ------------------------------------------------- epilogue (both CTAs)
         // Epilogue warp w drains TMEM lanes 32 * (w % 4) .. +31 (its quarter of
@@ -350,6 +357,7 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
         const int j0 = ((warp - kEpiWarp0) >> 2) * kEpiBlocks;
         const uint32_t acc_empty_leader = mapa(bar(kBarAccEmpty), 0);
         const uint32_t stage = sbase + kOffStage + (uint32_t)(warp - kEpiWarp0) * kEpiStageBytes;
+        const uint32_t shift = 4 + P.yscale;  // x rows are scaled by 16
         uint32_t acc_phase = 0, nchunk = 0;
         bool ok = true;
         for (int u = first; u < last && ok; u++) {
@@ -366,10 +374,8 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
             const bool add = U.split || P.accumulate;
             const CUtensorMap *omap = P.use_param_map ? &pomap : &cd->omap;
             const int row0 = cd->orow + (int)(U.out_off >> 6);
-            if (!mbar_wait(bar(kBarAccFull), acc_phase, abort_flag)) {
-                ok = false;
-                break;
-            }
+            ok = mbar_wait_warp(bar(kBarAccFull), acc_phase, abort_flag);
+            if (!ok) break;
             acc_phase ^= 1;
             tc_fence_after();
 #pragma unroll 1
@@ -393,8 +399,8 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
                         tmem_wait_ld();
 #pragma unroll
                         for (int k = 0; k < 8; k++) {
-                            re[k] = (uint32_t)((int32_t)re[k] >> 4);
-                            im[k] = (uint32_t)((int32_t)im[k] >> 4);
+                            re[k] = (uint32_t)((int32_t)re[k] >> shift);
+                            im[k] = (uint32_t)((int32_t)im[k] >> shift);
                             if (!P.ut) im[k] = 0u - im[k];
                         }
                         stage_row_half(tile, lane, part, re, im);
@@ -416,7 +422,7 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(acc_empty_leader);
         }
-        if (!ok) {
+        if (!ok && lane == 0) {
             atomicOr(P.err, 0x800);
             *abort_flag = 1;
         }
@@ -456,6 +462,7 @@ cudaError_t launch_pair_map(const TcLaunch &L, const CUtensorMap *pmap, const CU
     P.use_param_map = L.use_param_map;
     P.ut = L.ut;
     P.accumulate = L.accumulate;
+    P.yscale = L.max_samples <= kScaledMaxSamples ? 3 : 0;
     P.err = L.err;
     CUtensorMap dummy;
     memset(&dummy, 0, sizeof(dummy));
