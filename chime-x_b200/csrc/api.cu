@@ -111,11 +111,9 @@ int run_tc(chx_plan *p, const uint8_t *d_packed, int32_t *d_blocks, int map, int
         return fail(CHX_E_INVALID, "packed input must be 16-byte aligned for TMA");
     if ((reinterpret_cast<uintptr_t>(d_blocks) & 15) != 0)
         return fail(CHX_E_INVALID, "block buffer must be 16-byte aligned for TMA");
-    CUtensorMap tmap, omap;
-    int r = tc_encode_map(&tmap, d_packed, p->E, p->F, p->T, p->E, (int64_t)p->F * p->E);
+    TcMaps maps;
+    const int r = tc_encode_maps(&maps, d_packed, p->E, p->F, p->T, d_blocks);
     if (r != 0) return fail(CHX_E_CUDA, "cuTensorMapEncodeTiled failed (%d)", r);
-    r = tc_encode_out_map(&omap, d_blocks, (int64_t)p->F * p->NB * 32);
-    if (r != 0) return fail(CHX_E_CUDA, "cuTensorMapEncodeTiled (blocks) failed (%d)", r);
     if (p->has_split_units && !accumulate)
         CHX_CUDA(cudaMemsetAsync(d_blocks, 0, (size_t)chx_plan_block_words(p) * 4, st));
     TcLaunch L;
@@ -131,7 +129,7 @@ int run_tc(chx_plan *p, const uint8_t *d_packed, int32_t *d_blocks, int map, int
     L.accumulate = accumulate;
     L.err = p->d_err;
     L.grid = p->grid;
-    CHX_CUDA(tc_tile_launch(p->tile_built, L, &tmap, &omap, st));
+    CHX_CUDA(tc_tile_launch(p->tile_built, L, &maps, st));
     return CHX_OK;
 }
 

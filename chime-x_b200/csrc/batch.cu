@@ -114,7 +114,7 @@ int record_batch(chx_batch *b, cudaStream_t st, int accumulate) {
     L.accumulate = accumulate;
     L.err = b->d_err;
     L.grid = b->grid;
-    CHX_CUDA(tc_tile_launch(b->tile, L, nullptr, nullptr, st));
+    CHX_CUDA(tc_tile_launch(b->tile, L, nullptr, st));
     return CHX_OK;
 }
 
@@ -190,7 +190,10 @@ int chx_batch_create(chx_batch **out, int n, const chx_channel_desc *descs, int 
     // short integrations are not).  The autotuner's split was timed on a lone
     // channel, where splitting fills idle SMs that a batch already fills, so
     // batches take only its tile.
-    const int auto_split = tc_choose_split(b->tile, sm_count, [&](int k, std::vector<Unit> &u) {
+    int64_t out_bytes = 0;
+    for (int c = 0; c < n; c++)
+        out_bytes += descs[c].num_integrations * num_blocks_of(descs[c].num_elements) * 8192;
+    const int auto_split = tc_choose_split(b->tile, sm_count, out_bytes, [&](int k, std::vector<Unit> &u) {
         for (int c = 0; c < n; c++)
             for (int i = 0; i < descs[c].num_integrations; i++)
                 tc_append_tile_units(b->tile, u, c, descs[c].num_elements,
@@ -205,8 +208,12 @@ int chx_batch_create(chx_batch **out, int n, const chx_channel_desc *descs, int 
         const chx_channel_desc &d = descs[c];
         const int64_t stride = d.input_stride ? d.input_stride : d.num_elements;
         const int64_t samples = (int64_t)d.num_timesamples * d.num_integrations;
-        const int r = tc_encode_map(&chans[c].map, d.d_packed, d.num_elements, 1, samples,
-                                    ((int64_t)d.num_elements + 15) / 16 * 16, stride);
+        const int64_t chan_stride = ((int64_t)d.num_elements + 15) / 16 * 16;
+        int r = tc_encode_map(&chans[c].map, d.d_packed, d.num_elements, 1, samples, chan_stride,
+                              stride);
+        if (r == 0)
+            r = tc_encode_map(&chans[c].xmap, d.d_packed, d.num_elements, 1, samples, chan_stride,
+                              stride, 64);
         if (r != 0) {
             delete b;
             return fail(CHX_E_CUDA, "channel %d: cuTensorMapEncodeTiled failed (%d)", c, r);

@@ -114,7 +114,8 @@ cudaError_t launch_blocks_to_full(const int32_t *blocks, int32_t *full, int E, i
 // A channel as the tensor-core kernel sees it: the TMA map of its packed
 // samples (dims {E, channels, samples}), its block-buffer address and shape.
 struct __align__(64) ChanDesc {
-    CUtensorMap map;   // samples; used unless the launch passes one map for all channels
+    CUtensorMap map;   // samples (128-element tiles); used unless the launch passes one map for all channels
+    CUtensorMap xmap;  // samples in 64-element tiles (x of the SM-pair kernel); same rule
     CUtensorMap omap;  // block output as rows of 64 words (tc_encode_out_map); same rule
     uint64_t out;      // block buffer: absolute address, or byte offset added to
                        // the launch's out_base
@@ -124,7 +125,7 @@ struct __align__(64) ChanDesc {
     int orow;          // first row of this channel's blocks inside omap
     int pad[10];
 };
-static_assert(sizeof(ChanDesc) == 320, "ChanDesc layout");
+static_assert(sizeof(ChanDesc) == 448, "ChanDesc layout");
 
 // One work unit: a 128-element y tile against one or two 128-element x tiles
 // of one channel over samples [t0, t1).  tyx = ty | x0 << 10 | nx << 20.
@@ -134,22 +135,40 @@ struct Unit {
     int t0, t1;
     long long out_off;  // int32 words added to the channel's block buffer
     int split;          // 1: other units add to the same cells (TMA reduce-add)
-    int cost;           // samples x x-tiles, for scheduling
+    int cost;           // unit_cost, for scheduling
 };
 static_assert(sizeof(Unit) == 32, "Unit layout");
 
 constexpr int kUnitMaxSamples = 1 << 18;  // int32-exact bound per unit
 constexpr int kUnitStageSamples = 32;      // samples per pipeline stage of both kernels
 
-// Scheduling cost of a unit over samples [t0, t1): its pipeline stages, times
-// the x tiles it converts plus its y tile for the one-SM kernel (nx = 1 or 2
-// x tiles of 128 elements); SM-pair units all convert one y and one x tile per
-// SM, so their cost is their stage count.  Plans, batches, streams and the
+// Steps by which the SM-pair kernel's second x lane trails the first: about
+// one lane's accumulator drain.  8 to 14 measured within 1 % of each other
+// (E = 2048, T = 256 to 16384); below that the drains show again.
+constexpr int kSkewStages = 12;
+
+// Scheduling cost of a unit over samples [t0, t1), in cycles as measured with
+// clock64: nx x tiles of 128 elements against one y tile (one SM) or two (SM
+// pair).  SM pair: 512 per step of two lanes, 470 per step of one, at least the
+// lanes' drains of 4,700 each, and 1,500 of pipeline latency.  One SM: its
+// stages convert 1 + nx tiles at 330 cycles each, and every unit pays an
+// accumulator hand-off of about 16 stages.  Plans, batches, streams and the
 // allocation-free entry point share it so that their schedules agree.
 __host__ __device__ inline int unit_cost(bool pair, int t0, int t1, int nx) {
     const int stages = (t1 - t0 + kUnitStageSamples - 1) / kUnitStageSamples;
-    return pair ? stages : stages * (2 * nx + 1);
+    if (!pair) return (stages + 16) * (nx + 1) * 330;
+    const int skew = stages < kSkewStages ? stages : kSkewStages;
+    const int steps = nx < 2 ? 470 * stages : 512 * (stages - skew) + 2 * 470 * skew;
+    const int drain = 4700 * nx;
+    return (steps > drain ? steps : drain) + 1500;
 }
+
+// The TMA maps of a launch whose channels share them (TcLaunch::use_param_map).
+struct TcMaps {
+    CUtensorMap in;       // samples, 128-element tiles
+    CUtensorMap in_half;  // samples, 64-element tiles (x of the SM-pair kernel)
+    CUtensorMap out;      // blocks
+};
 
 struct TcLaunch {
     const ChanDesc *chans;  // device
@@ -173,38 +192,38 @@ void tc_append_units(std::vector<Unit> &out, int chan, int E, int t_begin, int t
 // Assigns units to `grid` persistent CTAs (longest first, to the least
 // loaded CTA) and reorders them CTA by CTA; offsets gets grid + 1 entries.
 void tc_schedule(std::vector<Unit> &u, int grid, std::vector<int> &offsets);
-// Makespan, in unit-cost units, of that assignment when every unit also pays
-// `handoff_stages` of its stages for the accumulator hand-off.
-long long tc_estimate_makespan(const std::vector<Unit> &u, int grid, int handoff_stages);
+// Makespan of that assignment, in cycles.
+long long tc_estimate_makespan(const std::vector<Unit> &u, int grid);
 // Samples of the longest unit.
 int tc_max_samples(const std::vector<Unit> &u);
 // Number of sample-range splits k (1-8) whose units, made by build(k, out),
-// have the shortest estimated makespan on the tile variant.
-int tc_choose_split(int tile, int sm_count,
+// have the shortest estimated makespan on the tile variant; out_bytes: the
+// output that a split has to zero first.
+int tc_choose_split(int tile, int sm_count, int64_t out_bytes,
                     const std::function<void(int, std::vector<Unit> &)> &build);
 // The same for F channels of E elements and T samples.
 int tc_auto_split(int tile, int E, int F, int T, int sm_count);
 // Encodes the TMA map of packed samples: dims {E, channels, samples}.
+// box_elements elements x 32 samples per tile.
 int tc_encode_map(CUtensorMap *m, const void *base, int E, int channels, int64_t samples,
-                  int64_t chan_stride, int64_t sample_stride);
+                  int64_t chan_stride, int64_t sample_stride, int box_elements = 128);
 // Encodes the TMA map of a block buffer seen as `rows` rows of 64 int32 words
 // (one 32-cell block row of Re/Im pairs), tile {32 words, 32 rows}, 128-byte
 // swizzle.  The epilogues store (or add) their tiles through it.  rows must
 // stay below 2^31 (tc_out_rows_ok).
 int tc_encode_out_map(CUtensorMap *m, void *base, int64_t rows);
 inline bool tc_out_rows_ok(int64_t rows) { return rows > 0 && rows < (1LL << 31); }
-// param_map / param_omap: the maps every channel uses when L.use_param_map.
-cudaError_t tc_launch(const TcLaunch &L, const CUtensorMap *param_map,
-                      const CUtensorMap *param_omap, cudaStream_t st);
+// maps: the maps every channel uses when L.use_param_map.
+cudaError_t tc_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st);
 
 // ---- 2-SM tensor-core kernel (tc_pair_correlator.cu) ----
-// Units of 256 x 256 elements (tyx = ty2 | tx2 << 10, 128-element tile pairs),
+// Units of 256 x 256 elements (tyx = ty2 | tx2 << 10 | nl << 20: 128-element
+// tile pairs, nl = 1 where the second x tile lies outside the matrix, else 2),
 // computed by a cluster of two CTAs with tcgen05.mma.cta_group::2.  In the
 // launch, grid counts clusters and cta_offsets is indexed by cluster.
 void tc_append_pair_units(std::vector<Unit> &out, int chan, int E, int t_begin, int t_end,
                           int tsplit, long long out_off);
-cudaError_t tc_pair_launch(const TcLaunch &L, const CUtensorMap *param_map,
-                           const CUtensorMap *param_omap, cudaStream_t st);
+cudaError_t tc_pair_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st);
 
 // Tensor-core tile variants (CHX_OPT_TILE).
 constexpr int kTile1Sm = 1;  // 128 x 256 elements per CTA
@@ -216,8 +235,10 @@ int tc_default_tile(int E);
 void tc_append_tile_units(int tile, std::vector<Unit> &out, int chan, int E, int t_begin,
                           int t_end, int tsplit, long long out_off);
 int tc_tile_slots(int tile, int sm_count);
-cudaError_t tc_tile_launch(int tile, const TcLaunch &L, const CUtensorMap *param_map,
-                           const CUtensorMap *param_omap, cudaStream_t st);
+cudaError_t tc_tile_launch(int tile, const TcLaunch &L, const TcMaps *maps, cudaStream_t st);
+// Encodes a launch's shared maps for F channels of E elements and T samples
+// with blocks at d_blocks; 0 or an error code.
+int tc_encode_maps(TcMaps *m, const void *d_packed, int E, int F, int T, void *d_blocks);
 // Device address of the error word of chx_correlate_noalloc on the current
 // device (noalloc.cu); the bounded-wait self-test writes it in mode 2.
 cudaError_t noalloc_error_word(int **out);

@@ -54,13 +54,13 @@ static_assert(kOffChans % alignof(ChanDesc) == 0 && kOffUnits % 16 == 0, "table 
 // Zero-initialised when the library's device code is loaded.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
-// Units of equal cost: `per_chan` units per channel and chunk (all units of
-// the SM-pair tile, or the one-SM tile's units with nx x tiles) over the
-// sample chunks [chunk0, chunk0 + nchunks) of kUnitMaxSamples samples.
+// Units of equal cost: `per_chan` units per channel and chunk, those with nx x
+// tiles (nx x lanes of the SM-pair tile), over the sample chunks
+// [chunk0, chunk0 + nchunks) of kUnitMaxSamples samples.
 struct UnitClass {
     int count;
     int chunk0, nchunks;
-    int nx;  // one-SM tile: 1 or 2 x tiles; SM-pair tile: 2
+    int nx;  // 1 or 2
     int per_chan;
 };
 
@@ -80,13 +80,16 @@ struct TableParams {
 // order tc_append_pair_units / tc_append_units enumerate them.
 __device__ int kth_tyx(const TableParams &P, int nx, int k) {
     if (P.pair) {
-        const int nt2 = (P.nt + 1) / 2;
+        // One lane: the last x tile pair of every row, when its second tile is
+        // missing.  Two lanes: the triangle of the full x tile pairs.
+        if (nx == 1) return k | ((P.nt / 2) << 10) | (1 << 20);
+        const int nt2 = P.nt / 2;
         int ty2 = 0;
         while (ty2 < nt2 - 1 && k >= nt2 - ty2) {
             k -= nt2 - ty2;
             ty2++;
         }
-        return ty2 | ((ty2 + k) << 10);
+        return ty2 | ((ty2 + k) << 10) | (2 << 20);
     }
     for (int ty = 0; ty < P.nt; ty++) {
         const int rem = P.nt - ty;  // x tiles at and right of the diagonal
@@ -195,22 +198,17 @@ int64_t unit_classes(int E, int F, int T, bool pair, TableParams *P) {
     P->chunks = chunks;
     P->pair = pair ? 1 : 0;
     P->nclass = 0;
-    int64_t per[2];
-    int kinds[2], nkinds;
+    int64_t per[2] = {0, 0};  // units with two x tiles (lanes), with one
+    const int kinds[2] = {2, 1}, nkinds = 2;
     if (pair) {
-        const int nt2 = (nt + 1) / 2;
-        per[0] = (int64_t)nt2 * (nt2 + 1) / 2;
-        kinds[0] = 2;
-        nkinds = 1;
+        const int64_t nt2 = nt / 2;
+        per[0] = nt2 * (nt2 + 1) / 2;
+        per[1] = nt % 2 ? nt2 + 1 : 0;
     } else {
-        per[0] = per[1] = 0;
         for (int ty = 0; ty < nt; ty++) {
-            per[0] += (nt - ty) / 2;  // units with two x tiles
-            per[1] += (nt - ty) % 2;  // units with one
+            per[0] += (nt - ty) / 2;
+            per[1] += (nt - ty) % 2;
         }
-        kinds[0] = 2;
-        kinds[1] = 1;
-        nkinds = 2;
     }
     int64_t total = 0;
     for (int part = 0; part < 2; part++) {  // full chunks, then the last chunk
@@ -308,11 +306,9 @@ extern "C" int chx_correlate_noalloc(const uint8_t *d_packed, int32_t *d_blocks,
     if (P.chunks > 1 && !accumulate)
         CHX_CUDA(cudaMemsetAsync(d_blocks, 0, (size_t)F * P.nb * 2048 * 4, st));
 
-    CUtensorMap tmap, omap;
-    int r = tc_encode_map(&tmap, d_packed, E, F, T, E, (int64_t)F * E);
+    TcMaps maps;
+    const int r = tc_encode_maps(&maps, d_packed, E, F, T, d_blocks);
     if (r != 0) return fail(CHX_E_CUDA, "cuTensorMapEncodeTiled failed (%d)", r);
-    r = tc_encode_out_map(&omap, d_blocks, (int64_t)F * P.nb * 32);
-    if (r != 0) return fail(CHX_E_CUDA, "cuTensorMapEncodeTiled (blocks) failed (%d)", r);
     unsigned char *dscr = static_cast<unsigned char *>(scratch);
     TcLaunch L;
     L.chans = reinterpret_cast<const ChanDesc *>(dscr + kOffChans);
@@ -327,7 +323,7 @@ extern "C" int chx_correlate_noalloc(const uint8_t *d_packed, int32_t *d_blocks,
     L.accumulate = accumulate ? 1 : 0;
     L.err = reinterpret_cast<int *>(dscr + kOffErr);
     L.grid = P.grid;
-    CHX_CUDA(tc_tile_launch(tile, L, &tmap, &omap, st));
+    CHX_CUDA(tc_tile_launch(tile, L, &maps, st));
     return CHX_OK;
 }
 

@@ -317,7 +317,8 @@ int chx_stream_admit(chx_stream *s, int E, int TA, int *channel_id) {
         return fail(CHX_E_ADMISSION, "allocation for the channel failed: %s", cudaGetErrorString(e));
     }
     ChanDesc &d = s->h_chans[cid];
-    const int r = tc_encode_map(&d.map, c.ring, E, 1, 2LL * TA, E, E);
+    int r = tc_encode_map(&d.map, c.ring, E, 1, 2LL * TA, E, E);
+    if (r == 0) r = tc_encode_map(&d.xmap, c.ring, E, 1, 2LL * TA, E, E, 64);
     if (r != 0) {
         cudaFree(c.ring);
         cudaFree(c.dumps);
@@ -491,7 +492,7 @@ int chx_stream_submit(chx_stream *s, int n, const int *ids, const uint8_t *const
         L.max_samples = tc_max_samples(units);
         L.cta_offsets = (const int *)((const char *)sl.dev + ub);
         L.grid = grid;
-        e = tc_pair_launch(L, nullptr, nullptr, st);
+        e = tc_pair_launch(L, nullptr, st);
     }
     if (e == cudaSuccess && !units1.empty()) {
         L.units = (const Unit *)((const char *)sl.dev + u1b0);
@@ -499,7 +500,7 @@ int chx_stream_submit(chx_stream *s, int n, const int *ids, const uint8_t *const
         L.max_samples = tc_max_samples(units1);
         L.cta_offsets = (const int *)((const char *)sl.dev + u1b0 + u1b);
         L.grid = grid1;
-        e = tc_launch(L, nullptr, nullptr, st);
+        e = tc_launch(L, nullptr, st);
     }
     if (e == cudaSuccess) e = cudaEventRecord(sl.done, st);
     if (e != cudaSuccess) {

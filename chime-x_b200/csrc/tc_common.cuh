@@ -135,6 +135,31 @@ __device__ __forceinline__ void tma_add_2d(const CUtensorMap *map, uint32_t src,
         "r"(x), "r"(y), "r"(src)
         : "memory");
 }
+// The same for a converged warp: the lane with lead = 1 issues the store (or
+// add) and commits it as a bulk group of its own.
+__device__ __forceinline__ void tma_out_2d(uint32_t lead, uint32_t add, const CUtensorMap *map,
+                                           uint32_t src, int x, int y) {
+    asm volatile(
+        "{\n\t.reg .pred q, a, s;\n\t"
+        "setp.ne.b32 q, %0, 0;\n\t"
+        "setp.ne.and.b32 a, %1, 0, q;\n\t"
+        "setp.eq.and.b32 s, %1, 0, q;\n\t"
+        "@s cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%2, {%4, %5}], [%3];\n\t"
+        "@a cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group"
+        " [%2, {%4, %5}], [%3];\n\t"
+        "@q cp.async.bulk.commit_group;\n\t}" ::"r"(lead),
+        "r"(add), "l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(x), "r"(y)
+        : "memory");
+}
+template <int N>
+__device__ __forceinline__ void bulk_wait_read_lead(uint32_t lead) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %0, 0;\n\t"
+        "@q cp.async.bulk.wait_group.read %1;\n\t}" ::"r"(lead),
+        "n"(N)
+        : "memory");
+}
 __device__ __forceinline__ void bulk_commit() {
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
@@ -154,6 +179,11 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t
     return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46) |
            ((uint64_t)2 << 61);
+}
+
+// The same with the 64-byte swizzle (layout type 4): 64-element rows.
+__device__ __forceinline__ uint64_t sdesc64(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
+    return sdesc(saddr, lbo, sbo) + ((uint64_t)2 << 61);
 }
 
 // Instruction descriptor: kind::i8, D = s32, A = signed int8, B signed or
@@ -288,6 +318,10 @@ __device__ __forceinline__ void yconv_scaled(const YScale &c, uint32_t w, uint32
 // Byte offset of 16-byte chunk g of row r (0..7) in a 128-byte-swizzled atom.
 __device__ __forceinline__ uint32_t swz(int r, int g) {
     return (uint32_t)(r * 128 + ((g ^ r) << 4));
+}
+// The same for chunk g (0..3) of a 64-byte-swizzled atom.
+__device__ __forceinline__ uint32_t swz64(int r, int g) {
+    return (uint32_t)(r * 64 + ((g ^ (r >> 1)) << 4));
 }
 
 

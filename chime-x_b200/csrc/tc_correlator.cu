@@ -445,8 +445,7 @@ tc_correlate_kernel(const __grid_constant__ CUtensorMap pmap,
 }
 
 template <int MAP>
-cudaError_t launch_map(const TcLaunch &L, const CUtensorMap *pmap, const CUtensorMap *pomap,
-                       cudaStream_t st) {
+cudaError_t launch_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t st) {
     // The shared-memory opt-in is a per-device function attribute.
     static bool attr_done[64] = {};
     int dev = 0;
@@ -469,10 +468,10 @@ cudaError_t launch_map(const TcLaunch &L, const CUtensorMap *pmap, const CUtenso
     P.ut = L.ut;
     P.accumulate = L.accumulate;
     P.err = L.err;
-    CUtensorMap dummy;
-    memset(&dummy, 0, sizeof(dummy));
-    tc_correlate_kernel<MAP><<<L.grid, kThreads, kSmemBytes, st>>>(
-        pmap ? *pmap : dummy, pomap ? *pomap : dummy, P);
+    TcMaps none;
+    memset(&none, 0, sizeof(none));
+    const TcMaps &m = maps ? *maps : none;
+    tc_correlate_kernel<MAP><<<L.grid, kThreads, kSmemBytes, st>>>(m.in, m.out, P);
     return cudaGetLastError();
 }
 
@@ -505,10 +504,16 @@ int tc_tile_slots(int tile, int sm_count) {
     return tile == kTile2Sm ? sm_count / 2 : sm_count;
 }
 
-cudaError_t tc_tile_launch(int tile, const TcLaunch &L, const CUtensorMap *param_map,
-                           const CUtensorMap *param_omap, cudaStream_t st) {
-    if (tile == kTile2Sm) return tc_pair_launch(L, param_map, param_omap, st);
-    return tc_launch(L, param_map, param_omap, st);
+cudaError_t tc_tile_launch(int tile, const TcLaunch &L, const TcMaps *maps, cudaStream_t st) {
+    if (tile == kTile2Sm) return tc_pair_launch(L, maps, st);
+    return tc_launch(L, maps, st);
+}
+
+int tc_encode_maps(TcMaps *m, const void *d_packed, int E, int F, int T, void *d_blocks) {
+    int r = tc_encode_map(&m->in, d_packed, E, F, T, E, (int64_t)F * E);
+    if (r == 0) r = tc_encode_map(&m->in_half, d_packed, E, F, T, E, (int64_t)F * E, 64);
+    if (r == 0) r = tc_encode_out_map(&m->out, d_blocks, F * num_blocks_of(E) * 32);
+    return r;
 }
 
 bool tc_supported(int E, int T) { return E >= 32 && E % 32 == 0 && E <= 65536 && T >= 1; }
@@ -584,13 +589,10 @@ int tc_max_samples(const std::vector<Unit> &u) {
     return m;
 }
 
-long long tc_estimate_makespan(const std::vector<Unit> &u, int grid, int handoff_stages) {
+long long tc_estimate_makespan(const std::vector<Unit> &u, int grid) {
     if (grid < 1) grid = 1;
     std::vector<long long> cost(u.size());
-    for (size_t i = 0; i < u.size(); i++) {
-        const long long st = std::max(1, (u[i].t1 - u[i].t0 + kStageSamples - 1) / kStageSamples);
-        cost[i] = u[i].cost + (long long)handoff_stages * u[i].cost / st;
-    }
+    for (size_t i = 0; i < u.size(); i++) cost[i] = u[i].cost;
     std::sort(cost.begin(), cost.end(), std::greater<long long>());
     std::priority_queue<long long, std::vector<long long>, std::greater<long long>> load;
     for (int b = 0; b < grid; b++) load.push(0);
@@ -604,18 +606,17 @@ long long tc_estimate_makespan(const std::vector<Unit> &u, int grid, int handoff
     return span;
 }
 
-int tc_choose_split(int tile, int sm_count,
+int tc_choose_split(int tile, int sm_count, int64_t out_bytes,
                     const std::function<void(int, std::vector<Unit> &)> &build) {
-    // A unit's accumulator hand-off costs about as much as 11 of its stages in
-    // the SM-pair kernel (measured on B200: ~9,400 cycles against ~850 per
-    // stage) and about 16 in the one-SM kernel, whose unpack warps run the
-    // epilogue themselves.  Splitting a channel's samples therefore pays only
-    // while it fills idle SMs.  With these overheads the estimate came within
-    // 2 % of the best measured split of every shape tried (E = 256-2048,
-    // F = 1-16, T = 16384; e.g. E = 1024, F = 2: 7 splits, 1551 vs 598 TOPS
-    // unsplit; E = 2048, F = 8: no split).  A split must win by 3 % to pay for
-    // zeroing the output and for the reduce-adds.
-    const int handoff_stages = tile == kTile2Sm ? 11 : 16;
+    // Every range of samples is a unit of its own, with its drain and pipeline
+    // latency (unit_cost), so splitting a channel's samples pays only while it
+    // fills idle SMs.  It also zeroes the output first: a launch of its own
+    // (about 5,500 cycles) and the bytes at about 2,600 a cycle.  Measured on
+    // B200 (us, unsplit / best split): E = 1024, F = 4, T = 1912 28.8 / 35.0 (3),
+    // E = 512, F = 1, T = 512 14.5 / 15.4 (7), E = 512, F = 8, T = 1024 20.6 / 18.7
+    // (3), E = 256, F = 16, T = 16384 148.6 / 51.4 (4), E = 640, F = 8, T = 16384
+    // 151.7 / 109.1 (3), E = 2048, F = 8, T = 16384 593.6 / 668.9 (2).
+    const long long zeroing = 5500 + out_bytes / 2600;
     const int grid_slots = tc_tile_slots(tile, sm_count);
     long long best = -1;
     int best_k = 1;
@@ -631,7 +632,7 @@ int tc_choose_split(int tile, int sm_count,
         if (units.size() == last_n) continue;
         last_n = units.size();
         const int grid = (int)std::min<size_t>(units.size(), (size_t)std::max(1, grid_slots));
-        const long long span = tc_estimate_makespan(units, grid, handoff_stages);
+        const long long span = tc_estimate_makespan(units, grid) + (k > 1 ? zeroing : 0);
         if (best < 0 || (k == 1 ? span < best : span * 100 < best * 97)) {
             best = span;
             best_k = k;
@@ -641,13 +642,13 @@ int tc_choose_split(int tile, int sm_count,
 }
 
 int tc_auto_split(int tile, int E, int F, int T, int sm_count) {
-    return tc_choose_split(tile, sm_count, [&](int k, std::vector<Unit> &units) {
+    return tc_choose_split(tile, sm_count, F * num_blocks_of(E) * 8192, [&](int k, std::vector<Unit> &units) {
         for (int f = 0; f < F; f++) tc_append_tile_units(tile, units, f, E, 0, T, k, 0);
     });
 }
 
 int tc_encode_map(CUtensorMap *m, const void *base, int E, int channels, int64_t samples,
-                  int64_t chan_stride, int64_t sample_stride) {
+                  int64_t chan_stride, int64_t sample_stride, int box_elements) {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
     if (!fn) {
         cudaDriverEntryPointQueryResult q;
@@ -660,7 +661,7 @@ int tc_encode_map(CUtensorMap *m, const void *base, int E, int channels, int64_t
     }
     cuuint64_t dims[3] = {(cuuint64_t)E, (cuuint64_t)channels, (cuuint64_t)samples};
     cuuint64_t strides[2] = {(cuuint64_t)chan_stride, (cuuint64_t)sample_stride};
-    cuuint32_t box[3] = {128, 1, (cuuint32_t)kStageSamples};
+    cuuint32_t box[3] = {(cuuint32_t)box_elements, 1, (cuuint32_t)kStageSamples};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void *>(base), dims, strides,
                     box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -690,15 +691,14 @@ int tc_encode_out_map(CUtensorMap *m, void *base, int64_t rows) {
     return r == CUDA_SUCCESS ? 0 : (int)r;
 }
 
-cudaError_t tc_launch(const TcLaunch &L, const CUtensorMap *param_map,
-                      const CUtensorMap *param_omap, cudaStream_t st) {
+cudaError_t tc_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st) {
     if (L.nunits <= 0) return cudaSuccess;
     if (L.grid <= 0) return cudaErrorInvalidValue;
-    if (L.use_param_map && (!param_map || !param_omap)) return cudaErrorInvalidValue;
+    if (L.use_param_map && !maps) return cudaErrorInvalidValue;
     switch (L.map) {
-    case MAP_EXACT: return launch_map<MAP_EXACT>(L, param_map, param_omap, st);
-    case MAP_CONF: return launch_map<MAP_CONF>(L, param_map, param_omap, st);
-    default: return launch_map<MAP_PACKED>(L, param_map, param_omap, st);
+    case MAP_EXACT: return launch_map<MAP_EXACT>(L, maps, st);
+    case MAP_CONF: return launch_map<MAP_CONF>(L, maps, st);
+    default: return launch_map<MAP_PACKED>(L, maps, st);
     }
 }
 
