@@ -65,13 +65,19 @@ cudaError_t build_tc_tables(chx_plan *p) {
     // if any, else the default; the split comes from the makespan estimate,
     // which sees how many units this plan has (the tuner times a workload that
     // fills the GPU, where splitting only adds hand-offs).
-    int tile = p->tile, split = p->tsplit;
+    int tile = p->tile;
     int tuned_tile = 0, tuned_split = 0;
     if (!tile && tc_tune_lookup(p->device, p->E, p->T, &tuned_tile, &tuned_split))
         tile = tuned_tile;
     if (!tile) tile = tc_default_tile(p->E);
-    if (!split) split = tc_auto_split(tile, p->E, p->F, p->T, p->sm_count);
-    for (int f = 0; f < p->F; f++) tc_append_tile_units(tile, units, f, p->E, 0, p->T, split, 0);
+    const TcShape shape =
+        tc_choose_shape(tile, p->tsplit, p->sm_count, p->F * p->NB * 8192,
+                        [&](TcShape s, std::vector<int> &costs) {
+                            tc_append_costs(s, p->E, p->T, p->F, costs);
+                        });
+    tile = shape.tile;
+    for (int f = 0; f < p->F; f++)
+        tc_append_tile_units(tile, units, f, p->E, 0, p->T, shape.split, 0);
     const int slots = tc_tile_slots(tile, p->sm_count);
     const int grid = (int)std::min<size_t>(units.size(), (size_t)std::max(1, slots));
     std::vector<int> offsets;

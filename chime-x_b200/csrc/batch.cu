@@ -193,13 +193,13 @@ int chx_batch_create(chx_batch **out, int n, const chx_channel_desc *descs, int 
     int64_t out_bytes = 0;
     for (int c = 0; c < n; c++)
         out_bytes += descs[c].num_integrations * num_blocks_of(descs[c].num_elements) * 8192;
-    const int auto_split = tc_choose_split(b->tile, sm_count, out_bytes, [&](int k, std::vector<Unit> &u) {
-        for (int c = 0; c < n; c++)
-            for (int i = 0; i < descs[c].num_integrations; i++)
-                tc_append_tile_units(b->tile, u, c, descs[c].num_elements,
-                                     i * descs[c].num_timesamples,
-                                     (i + 1) * descs[c].num_timesamples, k, 0);
-    });
+    const TcShape shape = tc_choose_shape(
+        b->tile, 0, sm_count, out_bytes, [&](TcShape sh, std::vector<int> &costs) {
+            for (int c = 0; c < n; c++)
+                tc_append_costs(sh, descs[c].num_elements, descs[c].num_timesamples,
+                                descs[c].num_integrations, costs);
+        });
+    b->tile = shape.tile;
 
     std::vector<ChanDesc> chans(n);
     memset(chans.data(), 0, chans.size() * sizeof(ChanDesc));
@@ -229,12 +229,11 @@ int chx_batch_create(chx_batch **out, int n, const chx_channel_desc *descs, int 
         chans[c].E = d.num_elements;
         chans[c].nb1 = d.num_elements / 32;
         chans[c].fcoord = 0;
-        const int split = auto_split;
         const int64_t nb = num_blocks_of(d.num_elements);
         for (int i = 0; i < d.num_integrations; i++) {
             const size_t before = units.size();
             const int t0 = i * d.num_timesamples, t1 = t0 + d.num_timesamples;
-            tc_append_tile_units(b->tile, units, c, d.num_elements, t0, t1, split,
+            tc_append_tile_units(b->tile, units, c, d.num_elements, t0, t1, shape.split,
                                  (long long)i * nb * 2048);
             bool any_split = false;
             for (size_t k = before; k < units.size(); k++) any_split |= units[k].split != 0;

@@ -192,17 +192,21 @@ void tc_append_units(std::vector<Unit> &out, int chan, int E, int t_begin, int t
 // Assigns units to `grid` persistent CTAs (longest first, to the least
 // loaded CTA) and reorders them CTA by CTA; offsets gets grid + 1 entries.
 void tc_schedule(std::vector<Unit> &u, int grid, std::vector<int> &offsets);
-// Makespan of that assignment, in cycles.
-long long tc_estimate_makespan(const std::vector<Unit> &u, int grid);
 // Samples of the longest unit.
 int tc_max_samples(const std::vector<Unit> &u);
-// Number of sample-range splits k (1-8) whose units, made by build(k, out),
-// have the shortest estimated makespan on the tile variant; out_bytes: the
-// output that a split has to zero first.
-int tc_choose_split(int tile, int sm_count, int64_t out_bytes,
-                    const std::function<void(int, std::vector<Unit> &)> &build);
-// The same for F channels of E elements and T samples.
-int tc_auto_split(int tile, int E, int F, int T, int sm_count);
+// Makespan of that assignment, in cycles, from the units' costs (sorted here).
+long long tc_estimate_makespan(std::vector<int> &costs, int grid);
+// A tile variant and a number of sample-range splits.
+struct TcShape {
+    int tile, split;
+};
+// Shape whose units have the shortest estimated makespan: splits 1-8 (split = 0)
+// or the given one, wide or narrow units for the SM pair.  costs_of appends the
+// unit costs of a shape; out_bytes: the output that a split has to zero first.
+TcShape tc_choose_shape(int tile, int split, int sm_count, int64_t out_bytes,
+                        const std::function<void(TcShape, std::vector<int> &)> &costs_of);
+// Appends the unit costs of `count` integrations of E elements and T samples.
+void tc_append_costs(TcShape shape, int E, int T, int count, std::vector<int> &costs);
 // Encodes the TMA map of packed samples: dims {E, channels, samples}.
 // box_elements elements x 32 samples per tile.
 int tc_encode_map(CUtensorMap *m, const void *base, int E, int channels, int64_t samples,
@@ -217,18 +221,20 @@ inline bool tc_out_rows_ok(int64_t rows) { return rows > 0 && rows < (1LL << 31)
 cudaError_t tc_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st);
 
 // ---- 2-SM tensor-core kernel (tc_pair_correlator.cu) ----
-// Units of 256 x 256 elements (tyx = ty2 | tx2 << 10 | nl << 20: 128-element
-// tile pairs, nl = 1 where the second x tile lies outside the matrix, else 2),
-// computed by a cluster of two CTAs with tcgen05.mma.cta_group::2.  In the
-// launch, grid counts clusters and cta_offsets is indexed by cluster.
-void tc_append_pair_units(std::vector<Unit> &out, int chan, int E, int t_begin, int t_end,
-                          int tsplit, long long out_off);
+// Units of 256 y x (128 nl) x elements (tyx = ty2 | tx << 10 | nl << 20: a pair of
+// 128-element y tiles, the first of nl x tiles), computed by a cluster of two
+// CTAs with tcgen05.mma.cta_group::2; nl = 2, or 1 where the second x tile lies
+// outside the matrix and in narrow units.  In the launch, grid counts clusters
+// and cta_offsets is indexed by cluster.
+void tc_append_pair_units(std::vector<Unit> &out, bool narrow, int chan, int E, int t_begin,
+                          int t_end, int tsplit, long long out_off);
 cudaError_t tc_pair_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st);
 
 // Tensor-core tile variants (CHX_OPT_TILE).
 constexpr int kTile1Sm = 1;  // 128 x 256 elements per CTA
 constexpr int kTile2Sm = 2;  // 256 x 256 elements per CTA pair
-constexpr int kTileMax = kTile2Sm;
+constexpr int kTileMax = kTile2Sm;  // last one that a caller can choose
+constexpr int kTileNarrow = 3;      // SM pair with narrow units (tc_choose_shape)
 int tc_default_tile(int E);
 // Dispatch by tile variant: units of one channel's sample range, persistent
 // CTAs (or clusters) for `sm_count` SMs, and the launch.

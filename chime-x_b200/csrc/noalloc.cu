@@ -67,6 +67,7 @@ struct UnitClass {
 struct TableParams {
     int E, F, T;
     int pair;    // 1: SM-pair tile, 0: one-SM tile
+    int narrow;  // SM pair: units of one x tile
     int nt;      // 128-element tiles per channel
     int chunks;  // sample chunks
     int n;       // units
@@ -80,16 +81,16 @@ struct TableParams {
 // order tc_append_pair_units / tc_append_units enumerate them.
 __device__ int kth_tyx(const TableParams &P, int nx, int k) {
     if (P.pair) {
-        // One lane: the last x tile pair of every row, when its second tile is
-        // missing.  Two lanes: the triangle of the full x tile pairs.
-        if (nx == 1) return k | ((P.nt / 2) << 10) | (1 << 20);
-        const int nt2 = P.nt / 2;
-        int ty2 = 0;
-        while (ty2 < nt2 - 1 && k >= nt2 - ty2) {
-            k -= nt2 - ty2;
+        // Narrow: every x tile from the y pair's first one on.  Wide, one lane:
+        // the last x tile of every row, when the tile count is odd; two lanes:
+        // the x tile pairs.
+        if (nx == 1 && !P.narrow) return k | ((P.nt - 1) << 10) | (1 << 20);
+        int ty2 = 0, n;
+        while (k >= (n = P.narrow ? P.nt - 2 * ty2 : P.nt / 2 - ty2)) {
+            k -= n;
             ty2++;
         }
-        return ty2 | ((ty2 + k) << 10) | (2 << 20);
+        return ty2 | ((2 * ty2 + (P.narrow ? k : 2 * k)) << 10) | (nx << 20);
     }
     for (int ty = 0; ty < P.nt; ty++) {
         const int rem = P.nt - ty;  // x tiles at and right of the diagonal
@@ -191,19 +192,21 @@ cudaError_t scratch_address(int dev, void **out) {
 }
 
 // The unit classes of a call, in decreasing cost; returns the unit count.
-int64_t unit_classes(int E, int F, int T, bool pair, TableParams *P) {
+int64_t unit_classes(int E, int F, int T, int tile, TableParams *P) {
+    const bool pair = tile != kTile1Sm, narrow = tile == kTileNarrow;
     const int nt = (E + 127) / 128;
     const int chunks = (T + kUnitMaxSamples - 1) / kUnitMaxSamples;
     P->nt = nt;
     P->chunks = chunks;
     P->pair = pair ? 1 : 0;
+    P->narrow = narrow ? 1 : 0;
     P->nclass = 0;
     int64_t per[2] = {0, 0};  // units with two x tiles (lanes), with one
     const int kinds[2] = {2, 1}, nkinds = 2;
     if (pair) {
-        const int64_t nt2 = nt / 2;
-        per[0] = nt2 * (nt2 + 1) / 2;
-        per[1] = nt % 2 ? nt2 + 1 : 0;
+        const int64_t nt2 = nt / 2, wide = nt2 * (nt2 + 1) / 2, odd = nt % 2 ? nt2 + 1 : 0;
+        per[0] = narrow ? 0 : wide;
+        per[1] = narrow ? 2 * wide + odd : odd;
     } else {
         for (int ty = 0; ty < nt; ty++) {
             per[0] += (nt - ty) / 2;
@@ -277,19 +280,18 @@ extern "C" int chx_correlate_noalloc(const uint8_t *d_packed, int32_t *d_blocks,
     if (F > kNoAllocMaxChannels)
         return fail(CHX_E_UNSUPPORTED, "no-allocation entry point takes at most %d channels (F=%d)",
                     kNoAllocMaxChannels, F);
-    const int tile = tc_default_tile(E);
+    int tile = tc_default_tile(E);
     TableParams P;
     P.E = E;
     P.F = F;
     P.T = T;
     P.nb = num_blocks_of(E);
-    const int64_t nunits = unit_classes(E, F, T, tile == kTile2Sm, &P);
+    int64_t nunits = unit_classes(E, F, T, tile, &P);
     if (nunits > kNoAllocMaxUnits)
         return fail(CHX_E_UNSUPPORTED,
                     "no-allocation entry point takes at most %d work units; E=%d F=%d T=%d needs "
                     "%lld",
                     kNoAllocMaxUnits, E, F, T, (long long)nunits);
-    P.n = (int)nunits;
 
     int dev = 0;
     CHX_CUDA(cudaGetDevice(&dev));
@@ -297,7 +299,22 @@ extern "C" int chx_correlate_noalloc(const uint8_t *d_packed, int32_t *d_blocks,
     CHX_CUDA(scratch_address(dev, &scratch));
     int sm_count = 0;
     CHX_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev));
-    P.grid = std::min(std::min(P.n, tc_tile_slots(tile, sm_count)), kNoAllocMaxGrid);
+    const int slots = std::max(1, tc_tile_slots(tile, sm_count));
+    // Few units: narrow ones if their rounds are shorter (as tc_choose_shape).
+    if (tile == kTile2Sm && nunits < 2 * slots) {
+        TableParams N = P;
+        const int64_t nnarrow = unit_classes(E, F, T, kTileNarrow, &N);
+        auto span = [&](int64_t n, int nx) {
+            return (n + slots - 1) / slots * unit_cost(true, 0, std::min(T, kUnitMaxSamples), nx);
+        };
+        if (span(nnarrow, 1) * 100 < span(nunits, 2) * 97) {
+            tile = kTileNarrow;
+            nunits = nnarrow;
+            P = N;
+        }
+    }
+    P.n = (int)nunits;
+    P.grid = std::min(std::min(P.n, slots), kNoAllocMaxGrid);
 
     cudaStream_t st = (cudaStream_t)stream;
     const int threads = std::max(std::max(P.n, P.grid + 1), F);

@@ -284,8 +284,8 @@ int chx_stream_admit(chx_stream *s, int E, int TA, int *channel_id) {
     // The tile variant the plain path would choose for this E.
     const bool pair = tc_default_tile(E) == kTile2Sm;
     if (pair) {
-        tc_append_pair_units(u0, cid, E, 0, TA, 1, 0);
-        tc_append_pair_units(u1, cid, E, TA, 2 * TA, 1, NB * 2048);
+        tc_append_pair_units(u0, false, cid, E, 0, TA, 1, 0);
+        tc_append_pair_units(u1, false, cid, E, TA, 2 * TA, 1, NB * 2048);
     } else {
         tc_append_units(u0, cid, E, 0, TA, 1, 0);
         tc_append_units(u1, cid, E, TA, 2 * TA, 1, NB * 2048);

@@ -494,18 +494,18 @@ int tc_default_tile(int E) {
 
 void tc_append_tile_units(int tile, std::vector<Unit> &out, int chan, int E, int t_begin,
                           int t_end, int tsplit, long long out_off) {
-    if (tile == kTile2Sm)
-        tc_append_pair_units(out, chan, E, t_begin, t_end, tsplit, out_off);
+    if (tile != kTile1Sm)
+        tc_append_pair_units(out, tile == kTileNarrow, chan, E, t_begin, t_end, tsplit, out_off);
     else
         tc_append_units(out, chan, E, t_begin, t_end, tsplit, out_off);
 }
 
 int tc_tile_slots(int tile, int sm_count) {
-    return tile == kTile2Sm ? sm_count / 2 : sm_count;
+    return tile == kTile1Sm ? sm_count : sm_count / 2;
 }
 
 cudaError_t tc_tile_launch(int tile, const TcLaunch &L, const TcMaps *maps, cudaStream_t st) {
-    if (tile == kTile2Sm) return tc_pair_launch(L, maps, st);
+    if (tile != kTile1Sm) return tc_pair_launch(L, maps, st);
     return tc_launch(L, maps, st);
 }
 
@@ -589,15 +589,13 @@ int tc_max_samples(const std::vector<Unit> &u) {
     return m;
 }
 
-long long tc_estimate_makespan(const std::vector<Unit> &u, int grid) {
+long long tc_estimate_makespan(std::vector<int> &costs, int grid) {
     if (grid < 1) grid = 1;
-    std::vector<long long> cost(u.size());
-    for (size_t i = 0; i < u.size(); i++) cost[i] = u[i].cost;
-    std::sort(cost.begin(), cost.end(), std::greater<long long>());
+    std::sort(costs.begin(), costs.end(), std::greater<int>());
     std::priority_queue<long long, std::vector<long long>, std::greater<long long>> load;
     for (int b = 0; b < grid; b++) load.push(0);
     long long span = 0;
-    for (long long c : cost) {
+    for (int c : costs) {
         const long long l = load.top() + c;
         load.pop();
         load.push(l);
@@ -606,8 +604,8 @@ long long tc_estimate_makespan(const std::vector<Unit> &u, int grid) {
     return span;
 }
 
-int tc_choose_split(int tile, int sm_count, int64_t out_bytes,
-                    const std::function<void(int, std::vector<Unit> &)> &build) {
+TcShape tc_choose_shape(int tile, int split, int sm_count, int64_t out_bytes,
+                        const std::function<void(TcShape, std::vector<int> &)> &costs_of) {
     // Every range of samples is a unit of its own, with its drain and pipeline
     // latency (unit_cost), so splitting a channel's samples pays only while it
     // fills idle SMs.  It also zeroes the output first: a launch of its own
@@ -616,35 +614,47 @@ int tc_choose_split(int tile, int sm_count, int64_t out_bytes,
     // E = 512, F = 1, T = 512 14.5 / 15.4 (7), E = 512, F = 8, T = 1024 20.6 / 18.7
     // (3), E = 256, F = 16, T = 16384 148.6 / 51.4 (4), E = 640, F = 8, T = 16384
     // 151.7 / 109.1 (3), E = 2048, F = 8, T = 16384 593.6 / 668.9 (2).
+    //
+    // Narrow SM-pair units (one x tile) cost more per tile than wide ones, but
+    // fill idle SM pairs without zeroing and halve a unit's drain; they are tried
+    // while the wide units make less than two waves.
     const long long zeroing = 5500 + out_bytes / 2600;
-    const int grid_slots = tc_tile_slots(tile, sm_count);
-    long long best = -1;
-    int best_k = 1;
+    const size_t slots = (size_t)std::max(1, tc_tile_slots(tile, sm_count));
+    TcShape best{tile, split ? split : 1};
+    long long best_span = -1;
     size_t last_n = 0;
-    for (int k = 1; k <= 8; k++) {
-        std::vector<Unit> units;
-        build(k, units);
-        if (units.empty()) return 1;
+    for (int k = split ? split : 1; k <= (split ? split : 8); k++) {
+        std::vector<int> costs;
+        costs_of(TcShape{tile, k}, costs);
+        const size_t n = costs.size();
         // Eight or more waves of unsplit units leave at most about an eighth
         // of a wave idle, less than the hand-offs that splitting adds.
-        if (k == 1 && units.size() >= (size_t)8 * std::max(1, grid_slots)) return 1;
+        if (n == 0 || (k == 1 && n >= 8 * slots)) return best;
         // Ranges are rounded to whole stages: skip splits that cut the same way.
-        if (units.size() == last_n) continue;
-        last_n = units.size();
-        const int grid = (int)std::min<size_t>(units.size(), (size_t)std::max(1, grid_slots));
-        const long long span = tc_estimate_makespan(units, grid) + (k > 1 ? zeroing : 0);
-        if (best < 0 || (k == 1 ? span < best : span * 100 < best * 97)) {
-            best = span;
-            best_k = k;
+        if (n == last_n) continue;
+        last_n = n;
+        for (int narrow = 0; narrow < (tile == kTile2Sm && n < 2 * slots ? 2 : 1); narrow++) {
+            const TcShape shape{narrow ? kTileNarrow : tile, k};
+            if (narrow) {
+                costs.clear();
+                costs_of(shape, costs);
+            }
+            const int grid = (int)std::min(costs.size(), slots);
+            const long long span = tc_estimate_makespan(costs, grid) + (k > 1 ? zeroing : 0);
+            if (best_span < 0 || span * 100 < best_span * 97) {
+                best_span = span;
+                best = shape;
+            }
         }
     }
-    return best_k;
+    return best;
 }
 
-int tc_auto_split(int tile, int E, int F, int T, int sm_count) {
-    return tc_choose_split(tile, sm_count, F * num_blocks_of(E) * 8192, [&](int k, std::vector<Unit> &units) {
-        for (int f = 0; f < F; f++) tc_append_tile_units(tile, units, f, E, 0, T, k, 0);
-    });
+void tc_append_costs(TcShape shape, int E, int T, int count, std::vector<int> &costs) {
+    std::vector<Unit> units;
+    tc_append_tile_units(shape.tile, units, 0, E, 0, T, shape.split, 0);
+    for (int i = 0; i < count; i++)
+        for (const Unit &u : units) costs.push_back(u.cost);
 }
 
 int tc_encode_map(CUtensorMap *m, const void *base, int E, int channels, int64_t samples,

@@ -3,7 +3,7 @@
 //
 // A cluster of two CTAs computes a 256 x 256-element unit: CTA r holds y tile
 // 2*ty2 + r (its 128 rows of A, M = 256 over the pair).  The unit's x range is
-// two lanes of 128 elements, x tiles 2*tx2 and 2*tx2 + 1; CTA r holds 64
+// two lanes of 128 elements, x tiles tx and tx + 1; CTA r holds 64
 // elements of each (its columns of B, N = 128 per lane over the pair).  One
 // elected thread of CTA 0 issues tcgen05.mma.cta_group::2; each SM's tensor core
 // reads only its own A rows and B columns from its own shared memory.  Lane h
@@ -28,7 +28,8 @@
 // 284 -> 272 us, T = 256 141 -> 130 us, T = 16384 unchanged.  Two full units of
 // half the width, with an accumulator buffer each, were bound by shared memory
 // (360-400 cycles per step instead of 256) and no faster at T = 1024.  A unit
-// whose second x tile lies outside the matrix (odd tile counts) has one lane only.
+// whose second x tile lies outside the matrix (odd tile counts) has one lane
+// only, and so have the narrow units of launches that leave SM pairs idle.
 //
 // Warps: 0-15 unpack, 16 TMA producer, 17 MMA issuer (CTA 0), 18-25 epilogue.
 // The epilogue warps drain each lane's accumulators when its last step is
@@ -225,7 +226,7 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
             const CUtensorMap *xmap = P.use_param_map ? &pxmap : &cd->xmap;
             const int fc = cd->fcoord;
             const int y = (2 * (U.tyx & 1023) + (int)rank) * 128;
-            const int x = ((U.tyx >> 10) & 1023) * 256 + (int)rank * 64;
+            const int x = ((U.tyx >> 10) & 1023) * 128 + (int)rank * 64;
             for (int k = 0; k < S.total; k++) {
                 ok = mbar_wait_warp(bar(kBarEmptyPk) + 8 * s, ph ^ 1, abort_flag);
                 if (!ok) break;
@@ -412,7 +413,12 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
                     }
                 fence_proxy_async();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(full_op_leader + 8 * os);
+                if (lane == 0) {
+                    if (rank == 0)
+                        mbar_arrive(bar(kBarFullOp) + 8 * os);
+                    else
+                        mbar_arrive_cluster(full_op_leader + 8 * os);
+                }
             }
             g += (uint32_t)S.total;
         }
@@ -444,7 +450,7 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
             const Unit U = P.units[u];
             const ChanDesc *cd = P.chans + U.chan;
             const int nl = (U.tyx >> 20) & 3;
-            const int bx0 = ((U.tyx >> 10) & 1023) * 8;
+            const int bx0 = ((U.tyx >> 10) & 1023) * 4;
             const int nb1 = cd->nb1;
             const int by = (2 * (U.tyx & 1023) + (int)rank) * 4 + q;
             // Split units (other units cover the same cells' other sample ranges)
@@ -561,9 +567,9 @@ cudaError_t launch_pair_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t 
 
 }  // namespace
 
-void tc_append_pair_units(std::vector<Unit> &out, int chan, int E, int t_begin, int t_end,
-                          int tsplit, long long out_off) {
-    const int nt = (E + 127) / 128, nt2 = (nt + 1) / 2;
+void tc_append_pair_units(std::vector<Unit> &out, bool narrow, int chan, int E, int t_begin,
+                          int t_end, int tsplit, long long out_off) {
+    const int nt = (E + 127) / 128, lanes = narrow ? 1 : 2;
     const int span = t_end - t_begin;
     if (span <= 0) return;
     int splits = tsplit < 1 ? 1 : tsplit;
@@ -571,13 +577,13 @@ void tc_append_pair_units(std::vector<Unit> &out, int chan, int E, int t_begin, 
     chunk = (chunk + kStageSamples - 1) / kStageSamples * kStageSamples;
     if (chunk > kUnitMaxSamples) chunk = kUnitMaxSamples;
     splits = (span + chunk - 1) / chunk;
-    for (int ty2 = 0; ty2 < nt2; ty2++)
-        for (int tx2 = ty2; tx2 < nt2; tx2++)
+    for (int ty2 = 0; 2 * ty2 < nt; ty2++)
+        for (int tx = 2 * ty2; tx < nt; tx += lanes)
             for (int s = 0; s < splits; s++) {
-                const int nl = std::min(2, nt - 2 * tx2);
+                const int nl = std::min(lanes, nt - tx);
                 Unit u;
                 u.chan = chan;
-                u.tyx = ty2 | (tx2 << 10) | (nl << 20);
+                u.tyx = ty2 | (tx << 10) | (nl << 20);
                 u.t0 = t_begin + s * chunk;
                 u.t1 = std::min(t_end, u.t0 + chunk);
                 u.out_off = out_off;

@@ -54,3 +54,38 @@ def test_longest_scaled_unit_offset_maps(cx, kb, T):
     out = p.corr_compat(torch.from_numpy(packed).cuda(), zero)
     p.check_device()
     np.testing.assert_array_equal(out.cpu().numpy(), orc.corr_partials(packed, T, F, E, kb, 1))
+
+
+@pytest.mark.parametrize("E,F,T", [
+    (2048, 1, 1), (2048, 1, 33),          # fewer steps than the lanes' skew
+    (256, 3, 384), (256, 3, 416),         # as many steps as the skew, one more
+    (384, 2, 500), (1152, 1, 700),        # odd tile counts: one-lane units
+    (160, 2, 64), (512, 9, 1000),         # few units: narrow ones
+    (512, 40, 450), (384, 80, 450),       # several units per SM pair
+])
+@pytest.mark.parametrize("tsplit", [0, 1, 2])
+def test_skewed_lanes(cx, E, F, T, tsplit):
+    """Lane 1 trails lane 0 and wraps around the samples; every channel word
+    for word, through the plan, then added once more."""
+    packed = orc.generate(T, F, E, 4, 500 + E + T, no_repeat=1)
+    ref = np.concatenate([orc.correlate_channel(packed, T, F, E, f, 1) for f in range(F)])
+    p = pair_plan(cx, E, F, T, tsplit=tsplit)
+    d = torch.from_numpy(packed).cuda()
+    out = p.correlate(d)
+    np.testing.assert_array_equal(out.cpu().numpy(), ref)
+    p.correlate(d, out, accumulate=True)
+    p.check_device()
+    np.testing.assert_array_equal(out.cpu().numpy(), (ref.astype(np.int64) * 2).astype(np.int32))
+
+
+@pytest.mark.parametrize("E,F,T", [(256, 1, 40), (384, 2, 70), (512, 8, 1024), (1152, 3, 100),
+                                   (2048, 2, 64), (640, 40, 64)])
+def test_noalloc_narrow_and_wide_units(cx, E, F, T):
+    """The allocation-free entry point derives its units on the device: narrow
+    (few units) and wide ones, odd and even tile counts."""
+    packed = orc.generate(T, F, E, 4, 600 + E + T, no_repeat=1)
+    ref = np.concatenate([orc.correlate_channel(packed, T, F, E, f, 1) for f in range(F)])
+    out = torch.empty(ref.size, dtype=torch.int32, device="cuda")
+    cx.correlate_noalloc(torch.from_numpy(packed).cuda(), out, E, F, T)
+    cx.noalloc_check()
+    np.testing.assert_array_equal(out.cpu().numpy(), ref)
