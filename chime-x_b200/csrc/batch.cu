@@ -106,6 +106,7 @@ int record_batch(chx_batch *b, cudaStream_t st, int accumulate) {
     L.units = (const Unit *)b->d_units;
     L.nunits = b->nunits;
     L.max_samples = b->max_unit;
+    L.static_tables = 1;
     L.cta_offsets = (const int *)((const char *)b->d_units + (size_t)b->nunits * sizeof(Unit));
     L.out_base = 0;
     L.use_param_map = 0;

@@ -177,6 +177,7 @@ struct TcLaunch {
     int max_samples;        // samples of the longest unit
     const int *cta_offsets; // device, grid + 1 entries
     uint64_t out_base;      // added to ChanDesc::out
+    int static_tables = 0;  // 1: no work of the stream writes the tables
     int use_param_map;      // 1: every channel uses the kernel-parameter map
     int map;                // value map (MAP_*)
     int ut;

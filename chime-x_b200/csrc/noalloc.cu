@@ -104,6 +104,8 @@ __device__ int kth_tyx(const TableParams &P, int nx, int k) {
 // One thread per unit (and per channel descriptor and CTA offset): writes the
 // tables of one call into the scratch array.
 __global__ void noalloc_tables_kernel(const TableParams P) {
+    // the correlator kernel's launch and set-up overlap this kernel
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     unsigned char *scr = g_noalloc_scratch;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     ChanDesc *chans = reinterpret_cast<ChanDesc *>(scr + kOffChans);

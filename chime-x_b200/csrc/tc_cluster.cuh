@@ -26,17 +26,6 @@ __device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// One lane of a converged warp (the same one each time).
-__device__ __forceinline__ uint32_t elect_one() {
-    uint32_t p;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "elect.sync _|p, 0xffffffff;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(p));
-    return p;
-}
-
 // The loads of one step (packed y tile, the x tiles of lanes 0 and 1 where
 // act0 / act1 are set, channel fc, sample t) and the byte count its barrier
 // expects, issued by the lead lane.

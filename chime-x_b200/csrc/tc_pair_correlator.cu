@@ -138,6 +138,7 @@ struct KParams {
     int use_param_map;
     int ut;
     int accumulate;
+    int static_tables;  // the tables were complete before the launch
     uint32_t yscale;  // y rows are scaled by 2^yscale
     int *err;
 };
@@ -204,13 +205,21 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
+    // Set-up overlaps the previous kernel of the stream; tables that the stream
+    // itself writes are read only after that kernel.
+    if (!P.static_tables) pdl_wait();
+    const int first = P.cluster_offsets[cluster], last = P.cluster_offsets[cluster + 1];
+    if (warp == 0) {  // the first unit's records are on their way to L1 meanwhile
+        const int chan = first < last ? P.units[first].chan : 0;
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(&P.chans[chan].E));
+    }
     tc_fence_before();
     __syncthreads();
     cluster_sync();  // barriers of both CTAs initialised, TMEM allocated
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-
-    const int first = P.cluster_offsets[cluster], last = P.cluster_offsets[cluster + 1];
+    pdl_launch_dependents();
+    pdl_wait();
 
     if (warp == kProducerWarp) {
         // ------------------------------------------------- TMA producer (both CTAs)
@@ -508,7 +517,7 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
             atomicOr(P.err, 0x800);
             *abort_flag = 1;
         }
-        if (lead) bulk_wait_all();  // output tiles written
+        bulk_wait_read_lead<0>(lead);  // the staging tiles may go; the grid's end completes the writes
     }
 
     tc_fence_before();
@@ -543,6 +552,7 @@ cudaError_t launch_pair_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t 
     P.use_param_map = L.use_param_map;
     P.ut = L.ut;
     P.accumulate = L.accumulate;
+    P.static_tables = L.static_tables;
     P.yscale = L.max_samples <= kScaledMaxSamples ? 3 : 0;
     P.err = L.err;
     TcMaps none;
@@ -553,13 +563,15 @@ cudaError_t launch_pair_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t 
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = kSmemBytes;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     e = cudaLaunchKernelEx(&cfg, tc_pair_kernel<MAP>, m.in, m.in_half, m.out, P);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
