@@ -127,6 +127,7 @@ int run_tc(chx_plan *p, const uint8_t *d_packed, int32_t *d_blocks, int map, int
     L.units = (const Unit *)p->d_units;
     L.nunits = p->nunits;
     L.max_samples = p->max_unit;
+    L.max_elements = p->E;
     L.static_tables = 1;
     L.cta_offsets = (const int *)((const char *)p->d_units + (size_t)p->nunits * sizeof(Unit));
     L.out_base = (uint64_t)d_blocks;

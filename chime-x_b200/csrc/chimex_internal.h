@@ -163,6 +163,13 @@ __host__ __device__ inline int unit_cost(bool pair, int t0, int t1, int nx) {
     return (steps > drain ? steps : drain) + 1500;
 }
 
+// The same for a channel of one 128-element tile (tc_small_correlator.cu): 400
+// per step, and the drains overlap the next unit's steps.
+__host__ __device__ inline int small_unit_cost(int t0, int t1) {
+    const int stages = (t1 - t0 + kUnitStageSamples - 1) / kUnitStageSamples;
+    return 400 * stages + 2000;
+}
+
 // The TMA maps of a launch whose channels share them (TcLaunch::use_param_map).
 struct TcMaps {
     CUtensorMap in;       // samples, 128-element tiles
@@ -177,6 +184,7 @@ struct TcLaunch {
     int max_samples;        // samples of the longest unit
     const int *cta_offsets; // device, grid + 1 entries
     uint64_t out_base;      // added to ChanDesc::out
+    int max_elements;       // elements of the largest channel
     int static_tables = 0;  // 1: no work of the stream writes the tables
     int use_param_map;      // 1: every channel uses the kernel-parameter map
     int map;                // value map (MAP_*)
@@ -201,7 +209,7 @@ long long tc_estimate_makespan(std::vector<int> &costs, int grid);
 struct TcShape {
     int tile, split;
 };
-// Shape whose units have the shortest estimated makespan: splits 1-8 (split = 0)
+// Shape whose units have the shortest estimated makespan: splits 1-32 (split = 0)
 // or the given one, wide or narrow units for the SM pair.  costs_of appends the
 // unit costs of a shape; out_bytes: the output that a split has to zero first.
 TcShape tc_choose_shape(int tile, int split, int sm_count, int64_t out_bytes,
@@ -218,8 +226,13 @@ int tc_encode_map(CUtensorMap *m, const void *base, int E, int channels, int64_t
 // stay below 2^31 (tc_out_rows_ok).
 int tc_encode_out_map(CUtensorMap *m, void *base, int64_t rows);
 inline bool tc_out_rows_ok(int64_t rows) { return rows > 0 && rows < (1LL << 31); }
-// maps: the maps every channel uses when L.use_param_map.
+// maps: the maps every channel uses when L.use_param_map.  Channels of one
+// 128-element tile only go to tc_small_launch.
 cudaError_t tc_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st);
+
+// ---- kernel for channels of at most 128 elements (tc_small_correlator.cu) ----
+constexpr int kSmallElements = 128;
+cudaError_t tc_small_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st);
 
 // ---- 2-SM tensor-core kernel (tc_pair_correlator.cu) ----
 // Units of 256 y x (128 nl) x elements (tyx = ty2 | tx << 10 | nl << 20: a pair of

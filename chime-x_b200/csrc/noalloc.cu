@@ -140,7 +140,7 @@ __global__ void noalloc_tables_kernel(const TableParams P) {
     u.t1 = min(P.T, u.t0 + kUnitMaxSamples);
     u.out_off = 0;
     u.split = P.chunks > 1 ? 1 : 0;
-    u.cost = unit_cost(P.pair != 0, u.t0, u.t1, C.nx);
+    u.cost = P.nt == 1 ? small_unit_cost(u.t0, u.t1) : unit_cost(P.pair != 0, u.t0, u.t1, C.nx);
     // round robin: sorted unit i is the (i / grid)-th unit of CTA i % grid
     const int b = i % P.grid;
     units[b * per_cta + min(b, extra) + i / P.grid] = u;
@@ -334,6 +334,7 @@ extern "C" int chx_correlate_noalloc(const uint8_t *d_packed, int32_t *d_blocks,
     L.units = reinterpret_cast<const Unit *>(dscr + kOffUnits);
     L.nunits = P.n;
     L.max_samples = std::min(T, kUnitMaxSamples);
+    L.max_elements = E;
     L.cta_offsets = reinterpret_cast<const int *>(dscr + kOffOffsets);
     L.out_base = (uint64_t)d_blocks;
     L.use_param_map = 1;

@@ -490,6 +490,7 @@ int chx_stream_submit(chx_stream *s, int n, const int *ids, const uint8_t *const
         L.units = (const Unit *)sl.dev;
         L.nunits = (int)units.size();
         L.max_samples = tc_max_samples(units);
+        L.max_elements = 65536;  // not looked at by the SM pair
         L.cta_offsets = (const int *)((const char *)sl.dev + ub);
         L.grid = grid;
         e = tc_pair_launch(L, nullptr, st);
@@ -498,6 +499,7 @@ int chx_stream_submit(chx_stream *s, int n, const int *ids, const uint8_t *const
         L.units = (const Unit *)((const char *)sl.dev + u1b0);
         L.nunits = (int)units1.size();
         L.max_samples = tc_max_samples(units1);
+        L.max_elements = kSmallElements;  // tc_default_tile: one tile
         L.cta_offsets = (const int *)((const char *)sl.dev + u1b0 + u1b);
         L.grid = grid1;
         e = tc_launch(L, nullptr, st);

@@ -485,8 +485,9 @@ cudaError_t launch_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t st) {
 // 1408 2051 / 1953, 1152 1903 / 1611, 896 1514 / 1473, 640 1418 / 1449,
 // 384 953 / 732, and 2048 2741 / 2133.  The SM pair is the default from two
 // tiles up; a single tile (E <= 128) would leave three quarters of its one
-// pair unit empty, so it goes to the one-SM kernel.  Both stay available as a
-// tile option and to the autotuner.
+// pair unit empty, so it goes to the one-SM tile.  Both stay available as a
+// tile option and to the autotuner.  A launch of the one-SM tile whose channels
+// all fit one 128-element tile runs tc_small_correlator.cu's kernel.
 int tc_default_tile(int E) {
     const int nt = (E + 127) / 128;
     return nt >= 2 ? kTile2Sm : kTile1Sm;
@@ -539,7 +540,7 @@ void tc_append_units(std::vector<Unit> &out, int chan, int E, int t_begin, int t
                 u.t1 = std::min(t_end, u.t0 + chunk);
                 u.out_off = out_off;
                 u.split = splits > 1 ? 1 : 0;
-                u.cost = unit_cost(false, u.t0, u.t1, nx);
+                u.cost = nt == 1 ? small_unit_cost(u.t0, u.t1) : unit_cost(false, u.t0, u.t1, nx);
                 out.push_back(u);
             }
         }
@@ -623,7 +624,12 @@ TcShape tc_choose_shape(int tile, int split, int sm_count, int64_t out_bytes,
     TcShape best{tile, split ? split : 1};
     long long best_span = -1;
     size_t last_n = 0;
-    for (int k = split ? split : 1; k <= (split ? split : 8); k++) {
+    // More than eight ranges only for launches that would still leave SMs idle
+    // (E = 128, F = 1, T = 16384: 20.6 us with 8, 14.4 with 16).
+    static const int ks[] = {1, 2, 3, 4, 5, 6, 7, 8, 12, 16, 24, 32};
+    for (int i = 0; i < (split ? 1 : (int)(sizeof(ks) / sizeof(ks[0]))); i++) {
+        const int k = split ? split : ks[i];
+        if (k > 8 && last_n >= slots) break;
         std::vector<int> costs;
         costs_of(TcShape{tile, k}, costs);
         const size_t n = costs.size();
@@ -705,6 +711,7 @@ cudaError_t tc_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st) {
     if (L.nunits <= 0) return cudaSuccess;
     if (L.grid <= 0) return cudaErrorInvalidValue;
     if (L.use_param_map && !maps) return cudaErrorInvalidValue;
+    if (L.max_elements <= kSmallElements) return tc_small_launch(L, maps, st);
     switch (L.map) {
     case MAP_EXACT: return launch_map<MAP_EXACT>(L, maps, st);
     case MAP_CONF: return launch_map<MAP_CONF>(L, maps, st);
