@@ -299,9 +299,8 @@ int chx_offset_accumulate(chx_plan *p, const uint8_t *d_packed, uint32_t *d_sums
         return fail(CHX_E_INVALID, "device buffers must be 16-byte aligned");
     DeviceGuard g(p->device);
     cudaStream_t st = (cudaStream_t)stream;
-    if (!accumulate)
-        CHX_CUDA(cudaMemsetAsync(d_sums, 0, (size_t)chx_plan_sum_words(p) * 4, st));
-    CHX_CUDA(launch_offset_accumulate(d_packed, d_sums, p->E, p->F, p->T, st));
+    if (!accumulate) CHX_CUDA(launch_zero(d_sums, chx_plan_sum_words(p) * 4, st));
+    CHX_CUDA(launch_offset_accumulate(d_packed, d_sums, p->E, p->F, p->T, !accumulate, st));
     return CHX_OK;
 }
 

@@ -101,8 +101,11 @@ inline int64_t num_blocks_of(int E) {
 cudaError_t launch_correlate_simt(const uint8_t *packed, int32_t *blocks, int E, int F,
                                   int T, int map, int ut, int mode, int splits,
                                   cudaStream_t st);
+// zeroed: launch_zero(sums) was the stream's previous launch.
 cudaError_t launch_offset_accumulate(const uint8_t *packed, uint32_t *sums, int E, int F,
-                                     int T, cudaStream_t st);
+                                     int T, bool zeroed, cudaStream_t st);
+// Zeroes bytes (a multiple of 16) at a 16-byte aligned address.
+cudaError_t launch_zero(void *out, int64_t bytes, cudaStream_t st);
 cudaError_t launch_preseed(const uint32_t *sums, int32_t *blocks, int E, int F, int T,
                            int packed_variant, int ut, cudaStream_t st);
 cudaError_t launch_blocks_to_triangle(const int32_t *blocks, int32_t *tri, int E, int F,

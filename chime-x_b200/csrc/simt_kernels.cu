@@ -163,23 +163,42 @@ correlate_simt_kernel(const uint8_t *__restrict__ packed, int32_t *__restrict__ 
         }
 }
 
+// Zeroes words of 16 bytes.  The next kernel may start meanwhile (programmatic
+// dependent launch) and waits before it adds to them.
+__global__ void zero_kernel(uint4 *out, int64_t n) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 // offsetAccumulateElements (offset_accumulator.cl:18-47).  The work is the
 // (vector block, 16-sample group) space: a vector block is 32 consecutive
 // 16-byte vectors of a sample row (16 (f, e) bytes each), a group 16 samples.
-// Each CTA takes an equal, contiguous share of that space (so every SM of the
-// single wave streams the same number of bytes); inside a share, warp w
-// streams the groups w, w + 8, ... of one vector block at a time (each lane
+// Each CTA (one of 16 warps per SM) takes an equal, contiguous share of that
+// space, so every SM streams the same number of bytes; inside a share, warp w
+// streams the groups w, w + 16, ... of one vector block at a time (each lane
 // one vector: coalesced 512-byte rows), loading a group's 16 vectors at once
-// so that enough bytes are in flight to keep HBM busy.  The nibbles are summed
-// four lanes at a time in byte-wide SWAR registers (15 * 16 < 256) and flushed
-// to 32-bit sums after every group; the 8 warps' sums meet in shared memory,
-// and the CTAs' in one atomic add per word for each vector block they touch.
-constexpr int kOaWarps = 8;
+// so that enough bytes are in flight to keep HBM busy (131 KiB per SM).  Four samples' words are
+// transposed so that a word holds four samples of one element, whose byte sum
+// (16 re + im) and low-nibble sum (im) are one dp4a each: three ALU instructions
+// per word and 32-bit sums throughout, where masking and adding nibbles in byte
+// lanes took six with the flushes.  The warps' sums meet in shared memory, and
+// the CTAs' in one atomic add per word for each vector block they touch, after
+// the kernel that zeroed the sums (zero_kernel) has ended.  Bound by HBM: with
+// the zeroing, E = 2048, F = 8, T = 16384 (268 MB) took 53.1 us with three CTAs of
+// 8 warps and byte-lane adds, 48.1 with dp4a and two CTAs, 45.4 with one CTA of
+// 16 warps (5.9 TB/s; the read alone 41 us at the copy rate); half as many bytes
+// in flight or twice as many CTAs measured slower.
+constexpr int kOaWarps = 16;
+constexpr int kOaMinGroups = 8;  // groups per CTA below which fewer CTAs are launched:
+                                 // their atomic adds cost more than their loads (E = 128,
+                                 // F = 5, T = 2968: 17.6 us with 1, 6.3 with 8)
 
-__global__ void __launch_bounds__(kOaWarps * 32)
+__global__ void __launch_bounds__(kOaWarps * 32, 1)
 offset_accumulate_kernel(const uint8_t *__restrict__ packed, uint32_t *__restrict__ sums,
                          int64_t nvec, int T, int64_t ngroups, int64_t nwork) {
-    __shared__ uint32_t part[kOaWarps][32][32];  // [warp][word][lane]
+    __shared__ uint32_t part[kOaWarps / 2][32][32];  // [warp pair][word][lane]
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint4 *p = reinterpret_cast<const uint4 *>(packed);
     const int64_t L1 = nwork * (blockIdx.x + 1) / gridDim.x;
@@ -188,54 +207,70 @@ offset_accumulate_kernel(const uint8_t *__restrict__ packed, uint32_t *__restric
         const int64_t end = min(L1, (vb + 1) * ngroups);  // this vector block's part
         const int64_t g0 = L - vb * ngroups, g1 = end - vb * ngroups;
         const int64_t i = vb * 32 + lane;
-        uint32_t s[32];  // element 4q + j: s[2 (4q + j)] re, s[2 (4q + j) + 1] im
+        uint32_t tot[16], lo[16];  // per element: sums of the bytes and of their low nibbles
 #pragma unroll
-        for (int k = 0; k < 32; k++) s[k] = 0u;
+        for (int k = 0; k < 16; k++) tot[k] = lo[k] = 0u;
         if (i < nvec) {
             for (int64_t g = g0 + w; g < g1; g += kOaWarps) {
                 const int t = (int)(16 * g);
-                uint32_t lo[4] = {0u, 0u, 0u, 0u}, hi[4] = {0u, 0u, 0u, 0u};
                 const uint4 *row = p + (int64_t)t * nvec + i;
-                auto add = [&](const uint4 v) {
-                    lo[0] += v.x & 0x0F0F0F0Fu;
-                    hi[0] += (v.x >> 4) & 0x0F0F0F0Fu;
-                    lo[1] += v.y & 0x0F0F0F0Fu;
-                    hi[1] += (v.y >> 4) & 0x0F0F0F0Fu;
-                    lo[2] += v.z & 0x0F0F0F0Fu;
-                    hi[2] += (v.z >> 4) & 0x0F0F0F0Fu;
-                    lo[3] += v.w & 0x0F0F0F0Fu;
-                    hi[3] += (v.w >> 4) & 0x0F0F0F0Fu;
-                };
+                uint4 v[16];
                 if (t + 16 <= T) {  // a full group: 16 independent loads in flight
-                    uint4 v[16];
 #pragma unroll
-                    for (int k = 0; k < 16; k++) v[k] = __ldg(row + (int64_t)k * nvec);
-#pragma unroll
-                    for (int k = 0; k < 16; k++) add(v[k]);
+                    for (int k = 0; k < 16; k++) v[k] = __ldcs(row + (int64_t)k * nvec);
                 } else {
-                    for (int k = 0; t + k < T; k++) add(__ldg(row + (int64_t)k * nvec));
+#pragma unroll
+                    for (int k = 0; k < 16; k++)
+                        v[k] = t + k < T ? __ldcs(row + (int64_t)k * nvec) : make_uint4(0, 0, 0, 0);
                 }
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
+                for (int k = 0; k < 16; k += 4) {
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        s[2 * (4 * q + j)] += (hi[q] >> (8 * j)) & 0xFFu;
-                        s[2 * (4 * q + j) + 1] += (lo[q] >> (8 * j)) & 0xFFu;
+                    for (int q = 0; q < 4; q++) {
+                        auto word = [&](int s) {
+                            const uint4 u = v[k + s];
+                            return q == 0 ? u.x : q == 1 ? u.y : q == 2 ? u.z : u.w;
+                        };
+                        const uint32_t a = word(0), b = word(1), c = word(2), e = word(3);
+                        const uint32_t ab0 = __byte_perm(a, b, 0x5140);  // a0 b0 a1 b1
+                        const uint32_t ab2 = __byte_perm(a, b, 0x7362);  // a2 b2 a3 b3
+                        const uint32_t ce0 = __byte_perm(c, e, 0x5140);
+                        const uint32_t ce2 = __byte_perm(c, e, 0x7362);
+                        const uint32_t x[4] = {
+                            __byte_perm(ab0, ce0, 0x5410), __byte_perm(ab0, ce0, 0x7632),
+                            __byte_perm(ab2, ce2, 0x5410), __byte_perm(ab2, ce2, 0x7632)};
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            tot[4 * q + j] = __dp4a(x[j], 0x01010101u, tot[4 * q + j]);
+                            lo[4 * q + j] = __dp4a(x[j] & 0x0F0F0F0Fu, 0x01010101u, lo[4 * q + j]);
+                        }
                     }
                 }
             }
         }
+        if (w < kOaWarps / 2)
 #pragma unroll
-        for (int k = 0; k < 32; k++) part[w][k][lane] = s[k];
+            for (int k = 0; k < 16; k++) {
+                part[w][2 * k][lane] = (tot[k] - lo[k]) >> 4;
+                part[w][2 * k + 1][lane] = lo[k];
+            }
         __syncthreads();
-        // Thread r handles (word, lane) pairs r, r + 256, ...: sum over the warps.
+        if (w >= kOaWarps / 2)
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                part[w - kOaWarps / 2][2 * k][lane] += (tot[k] - lo[k]) >> 4;
+                part[w - kOaWarps / 2][2 * k + 1][lane] += lo[k];
+            }
+        __syncthreads();
+        asm volatile("griddepcontrol.wait;" ::: "memory");  // the sums have been zeroed
+        // Thread r handles (word, lane) pairs r, r + 512: sum over the warps.
 #pragma unroll
         for (int r = threadIdx.x; r < 32 * 32; r += kOaWarps * 32) {
             const int k = r >> 5, l = r & 31;
             const int64_t iv = vb * 32 + l;
             uint32_t acc = 0u;
 #pragma unroll
-            for (int ww = 0; ww < kOaWarps; ww++) acc += part[ww][k][l];
+            for (int ww = 0; ww < kOaWarps / 2; ww++) acc += part[ww][k][l];
             if (iv < nvec && acc != 0u) atomicAdd(sums + 32 * iv + k, acc);
         }
         __syncthreads();  // part is rewritten for the next vector block
@@ -402,19 +437,37 @@ cudaError_t launch_correlate_simt(const uint8_t *packed, int32_t *blocks, int E,
 }
 
 cudaError_t launch_offset_accumulate(const uint8_t *packed, uint32_t *sums, int E, int F,
-                                     int T, cudaStream_t st) {
+                                     int T, bool zeroed, cudaStream_t st) {
     const int64_t nvec = (int64_t)F * E / 16;  // E % 32 == 0
     const int64_t vblocks = (nvec + 31) / 32;
     const int64_t ngroups = (T + 15) / 16;
     const int64_t nwork = vblocks * ngroups;
-    // One wave of three CTAs per SM (66 registers, 32 KiB shared memory), each
-    // with an equal share of the work.
+    // At most one CTA per SM, each with an equal share of the work.
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess)
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>((int64_t)3 * sms, nwork));
-    offset_accumulate_kernel<<<(unsigned)grid, kOaWarps * 32, 0, st>>>(packed, sums, nvec, T,
-                                                                      ngroups, nwork);
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(sms, nwork / kOaMinGroups));
+    // zeroed: the previous kernel of the stream is the one zeroing the sums; this
+    // one starts with it.  Otherwise an ordinary launch.
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(kOaWarps * 32);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = zeroed ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, offset_accumulate_kernel, packed, sums, nvec, T,
+                                       ngroups, nwork);
+    if (e != cudaSuccess) return e;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_zero(void *out, int64_t bytes, cudaStream_t st) {
+    const int64_t n = bytes / 16;
+    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(1184, (n + 1023) / 1024));
+    zero_kernel<<<grid, 256, 0, st>>>(static_cast<uint4 *>(out), n);
     return cudaGetLastError();
 }
 

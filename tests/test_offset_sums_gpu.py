@@ -1,0 +1,32 @@
+"""Offset sums at the edges of the kernel's work split, against the CPU oracle
+(integer sums: no tolerance)."""
+import numpy as np
+import pytest
+
+import pyoracle as orc
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("E,F,T", [
+    (32, 1, 1), (32, 1, 15), (32, 1, 17),         # one partial group, a group and one sample
+    (96, 3, 127), (96, 3, 129),                   # the fewest groups per CTA, one more
+    (512, 1, 2048), (544, 1, 2047),               # one vector block, a partial second one
+    (2048, 2, 3000), (1120, 5, 1111),             # shares crossing vector blocks
+])
+def test_offset_sums(E, F, T):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import chimex as cx
+    packed = orc.generate(T, F, E, 4, 50 + E + T, no_repeat=1)
+    packed[:E * F] = 0xFF
+    ref = orc.offset_accumulate(packed, T, F, E)
+    p = cx.Plan(E, F, T)
+    d = torch.from_numpy(packed).cuda()
+    sums = torch.full((p.sum_words,), -1, dtype=torch.int32, device="cuda")
+    for _ in range(3):  # each call zeroes first
+        p.offset_accumulate(d, sums)
+    np.testing.assert_array_equal(sums.cpu().numpy().view(np.uint32), ref)
+    p.offset_accumulate(d, sums, accumulate=True)
+    np.testing.assert_array_equal(sums.cpu().numpy().view(np.uint32), 2 * ref)
