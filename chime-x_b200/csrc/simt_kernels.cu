@@ -14,15 +14,17 @@ namespace chx {
 namespace {
 
 // (by, bx) of block b in the row-major upper-triangle enumeration of
-// main_wrapper.c:529-540.
+// main_wrapper.c:529-540: row y starts at block y nb1 - y (y - 1) / 2.  The root
+// of that quadratic, corrected for the float's rounding.
 __device__ __forceinline__ void decode_block(int b, int nb1, int &by, int &bx) {
-    int r = b, y = 0;
-    while (r >= nb1 - y) {
-        r -= nb1 - y;
-        y++;
-    }
+    auto start = [&](int y) { return y * nb1 - y * (y - 1) / 2; };
+    const float n = 2.0f * nb1 + 1.0f;
+    int y = (int)(0.5f * (n - sqrtf(fmaxf(n * n - 8.0f * (float)b, 0.0f))));
+    y = min(max(y, 0), nb1 - 1);
+    while (y > 0 && start(y) > b) y--;
+    while (y + 1 < nb1 && start(y + 1) <= b) y++;
     by = y;
-    bx = y + r;
+    bx = y + (b - start(y));
 }
 
 // Operand bytes of one packed sample under a value map (see chimex_internal.h).
@@ -344,41 +346,57 @@ preseed_kernel(const uint32_t *__restrict__ sums, int32_t *__restrict__ blocks, 
                           packed_variant, ut, tid);
 }
 
-// Block layout -> packed triangle (gpu_data_reorg.c:76-124).  The block is
-// read into shared memory with 16-byte loads; each of its rows is a
-// contiguous run of cells in the triangle (x >= y only on the diagonal
-// block) starting at any cell index, so every row is written as 16-byte
-// stores of cell pairs, with a single 8-byte store for an odd first cell and
-// for an odd last cell.  16 threads per row, two rows per thread.
+// Block layout -> packed triangle (gpu_data_reorg.c:76-124).  A CTA takes
+// kTriBlocks consecutive blocks: all are read into shared memory with 16-byte
+// loads first; each block row is a contiguous run of cells in the triangle
+// (x >= y only on the diagonal block) starting at any cell index, so every row
+// is written as 16-byte stores of cell pairs, with a single 8-byte store for an
+// odd first cell and for an odd last cell.  16 threads per row.  Both sides pass
+// through once, so loads and stores are marked streaming.  Bound by HBM: E = 2048,
+// F = 8 (271 MB) took 47.9 us with one block per CTA and plain accesses, 44.1 now
+// (6.1 TB/s); plain accesses with two blocks 44.4 (E = 1888: 38.2 against 37.0),
+// three blocks 44.8, four 52.4 (too few CTAs per SM).
+constexpr int kTriBlocks = 2;
+
 __global__ void __launch_bounds__(256)
 blocks_to_triangle_kernel(const int32_t *__restrict__ blocks, int32_t *__restrict__ tri,
                           int E, int nb1, int64_t nb) {
-    __shared__ __align__(16) int2 cells[32 * 32];
-    const int b = blockIdx.x, f = blockIdx.y;
-    int by, bx;
-    decode_block(b, nb1, by, bx);
+    __shared__ __align__(16) int2 cells[kTriBlocks][32 * 32];
+    const int b0 = blockIdx.x * kTriBlocks, f = blockIdx.y;
+    const int n = (int)min((int64_t)kTriBlocks, nb - b0);
     const int64_t ntri = (int64_t)E * (E + 1) / 2;
-    const int4 *blk = reinterpret_cast<const int4 *>(blocks + ((int64_t)f * nb + b) * 2048);
+    const int4 *blk = reinterpret_cast<const int4 *>(blocks + ((int64_t)f * nb + b0) * 2048);
     int4 *c4 = reinterpret_cast<int4 *>(cells);
+    int4 v[2 * kTriBlocks];
 #pragma unroll
-    for (int k = 0; k < 2; k++) c4[threadIdx.x + 256 * k] = __ldg(blk + threadIdx.x + 256 * k);
+    for (int k = 0; k < 2 * kTriBlocks; k++)
+        if (k < 2 * n) v[k] = __ldcs(blk + threadIdx.x + 256 * k);
+    int by, bx;
+    decode_block(b0, nb1, by, bx);
+#pragma unroll
+    for (int k = 0; k < 2 * kTriBlocks; k++)
+        if (k < 2 * n) c4[threadIdx.x + 256 * k] = v[k];
     __syncthreads();
+    for (int i = 0; i < n; i++) {
 #pragma unroll
-    for (int r = 0; r < 2; r++) {
-        const int slot = threadIdx.x + 256 * r, yl = slot >> 4, k = slot & 15;
-        const int xs = (bx == by) ? yl : 0;  // first cell of the row written
-        const int64_t y = by * 32 + yl;
-        const int64_t a0 = f * ntri + y * E - (y - 1) * y / 2 + (bx * 32 + xs - y);
-        const int head = (int)(a0 & 1);      // odd start: one 8-byte cell first
-        const int n = 32 - xs - head;        // cells after the head
-        const int2 *row = cells + yl * 32;
-        if (k < n / 2) {
-            const int x = xs + head + 2 * k;
-            const int2 u = row[x], v = row[x + 1];
-            *reinterpret_cast<int4 *>(tri + 2 * (a0 + head + 2 * k)) = make_int4(u.x, u.y, v.x, v.y);
+        for (int r = 0; r < 2; r++) {
+            const int slot = threadIdx.x + 256 * r, yl = slot >> 4, k = slot & 15;
+            const int xs = (bx == by) ? yl : 0;  // first cell of the row written
+            const int64_t y = by * 32 + yl;
+            const int64_t a0 = f * ntri + y * E - (y - 1) * y / 2 + (bx * 32 + xs - y);
+            const int head = (int)(a0 & 1);      // odd start: one 8-byte cell first
+            const int m = 32 - xs - head;        // cells after the head
+            const int2 *row = cells[i] + yl * 32;
+            if (k < m / 2) {
+                const int x = xs + head + 2 * k;
+                const int2 u = row[x], w = row[x + 1];
+                __stcs(reinterpret_cast<int4 *>(tri + 2 * (a0 + head + 2 * k)),
+                       make_int4(u.x, u.y, w.x, w.y));
+            }
+            if (k == 15 && head) *reinterpret_cast<int2 *>(tri + 2 * a0) = row[xs];
+            if (k == 14 && (m & 1)) *reinterpret_cast<int2 *>(tri + 2 * (a0 + 31 - xs)) = row[31];
         }
-        if (k == 15 && head) *reinterpret_cast<int2 *>(tri + 2 * a0) = row[xs];
-        if (k == 14 && (n & 1)) *reinterpret_cast<int2 *>(tri + 2 * (a0 + 31 - xs)) = row[31];
+        if (++bx == nb1) bx = ++by;  // the next block of the row, or the next row's diagonal
     }
 }
 
@@ -482,7 +500,7 @@ cudaError_t launch_preseed(const uint32_t *sums, int32_t *blocks, int E, int F, 
 
 cudaError_t launch_blocks_to_triangle(const int32_t *blocks, int32_t *tri, int E, int F,
                                       cudaStream_t st) {
-    dim3 grid((unsigned)num_blocks_of(E), (unsigned)F);
+    dim3 grid((unsigned)((num_blocks_of(E) + kTriBlocks - 1) / kTriBlocks), (unsigned)F);
     blocks_to_triangle_kernel<<<grid, 256, 0, st>>>(blocks, tri, E, E / 32, num_blocks_of(E));
     return cudaGetLastError();
 }
