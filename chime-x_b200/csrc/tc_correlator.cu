@@ -556,9 +556,26 @@ void tc_schedule(std::vector<Unit> &u, int grid, std::vector<int> &offsets) {
     // together read less (1.65x by sample range, then enumeration order) but
     // balance the CTAs worse and measured slower (1825 vs 2033 TOPS), and
     // ordering each CTA's units by channel read more (2.5x).
+    if (grid < 1) grid = 1;
+    // Units of one cost need no heap: the same assignment is round robin.  (A
+    // stream's submit schedules its units on the host every time.)
+    bool equal = true;
+    for (const Unit &x : u) equal &= x.cost == u[0].cost;
+    if (equal) {
+        const size_t n = u.size(), g = (size_t)grid;
+        offsets.resize(g + 1);
+        std::vector<Unit> out;
+        out.reserve(n);
+        for (size_t b = 0; b < g; b++) {
+            offsets[b] = (int)out.size();
+            for (size_t i = b; i < n; i += g) out.push_back(u[i]);
+        }
+        offsets[g] = (int)n;
+        u.swap(out);
+        return;
+    }
     std::stable_sort(u.begin(), u.end(),
                      [](const Unit &a, const Unit &b) { return a.cost > b.cost; });
-    if (grid < 1) grid = 1;
     std::vector<long long> load(grid, 0);
     std::vector<int> owner(u.size());
     std::vector<std::pair<long long, int>> heap;  // (load, cta), min-heap
