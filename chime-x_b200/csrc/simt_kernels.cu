@@ -351,11 +351,10 @@ preseed_kernel(const uint32_t *__restrict__ sums, int32_t *__restrict__ blocks, 
 // loads first; each block row is a contiguous run of cells in the triangle
 // (x >= y only on the diagonal block) starting at any cell index, so every row
 // is written as 16-byte stores of cell pairs, with a single 8-byte store for an
-// odd first cell and for an odd last cell.  16 threads per row.  Both sides pass
-// through once, so loads and stores are marked streaming.  Bound by HBM: E = 2048,
-// F = 8 (271 MB) took 47.9 us with one block per CTA and plain accesses, 44.1 now
-// (6.1 TB/s); plain accesses with two blocks 44.4 (E = 1888: 38.2 against 37.0),
-// three blocks 44.8, four 52.4 (too few CTAs per SM).
+// odd first cell and for an odd last cell.  16 threads per row.  Bound by HBM:
+// E = 2048, F = 8 (271 MB, three buffer sets in turn) took 48.0 us with one block
+// per CTA, 44.0 now (6.2 TB/s; a plain copy of as many bytes 45.1), 45.1 with three
+// blocks, 52.4 with four (too few CTAs per SM), 49.3 with streaming loads.
 constexpr int kTriBlocks = 2;
 
 __global__ void __launch_bounds__(256)
@@ -370,7 +369,7 @@ blocks_to_triangle_kernel(const int32_t *__restrict__ blocks, int32_t *__restric
     int4 v[2 * kTriBlocks];
 #pragma unroll
     for (int k = 0; k < 2 * kTriBlocks; k++)
-        if (k < 2 * n) v[k] = __ldcs(blk + threadIdx.x + 256 * k);
+        if (k < 2 * n) v[k] = __ldg(blk + threadIdx.x + 256 * k);
     int by, bx;
     decode_block(b0, nb1, by, bx);
 #pragma unroll
@@ -390,8 +389,8 @@ blocks_to_triangle_kernel(const int32_t *__restrict__ blocks, int32_t *__restric
             if (k < m / 2) {
                 const int x = xs + head + 2 * k;
                 const int2 u = row[x], w = row[x + 1];
-                __stcs(reinterpret_cast<int4 *>(tri + 2 * (a0 + head + 2 * k)),
-                       make_int4(u.x, u.y, w.x, w.y));
+                *reinterpret_cast<int4 *>(tri + 2 * (a0 + head + 2 * k)) =
+                    make_int4(u.x, u.y, w.x, w.y);
             }
             if (k == 15 && head) *reinterpret_cast<int2 *>(tri + 2 * a0) = row[xs];
             if (k == 14 && (m & 1)) *reinterpret_cast<int2 *>(tri + 2 * (a0 + 31 - xs)) = row[31];
