@@ -120,9 +120,11 @@ int run_tc(chx_plan *p, const uint8_t *d_packed, int32_t *d_blocks, int map, int
     TcMaps maps;
     const int r = tc_encode_maps(&maps, d_packed, p->E, p->F, p->T, d_blocks);
     if (r != 0) return fail(CHX_E_CUDA, "cuTensorMapEncodeTiled failed (%d)", r);
-    if (p->has_split_units && !accumulate)
-        CHX_CUDA(cudaMemsetAsync(d_blocks, 0, (size_t)chx_plan_block_words(p) * 4, st));
     TcLaunch L;
+    if (p->has_split_units && !accumulate) {
+        CHX_CUDA(launch_zero(d_blocks, chx_plan_block_words(p) * 4, st));
+        L.after_zero = 1;
+    }
     L.chans = (const ChanDesc *)p->d_chans;
     L.units = (const Unit *)p->d_units;
     L.nunits = p->nunits;

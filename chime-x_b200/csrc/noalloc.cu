@@ -105,7 +105,8 @@ __device__ int kth_tyx(const TableParams &P, int nx, int k) {
 // tables of one call into the scratch array.
 __global__ void noalloc_tables_kernel(const TableParams P) {
     // the correlator kernel's launch and set-up overlap this kernel
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_launch_dependents();
+    pdl_wait();
     unsigned char *scr = g_noalloc_scratch;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     ChanDesc *chans = reinterpret_cast<ChanDesc *>(scr + kOffChans);
@@ -320,8 +321,7 @@ extern "C" int chx_correlate_noalloc(const uint8_t *d_packed, int32_t *d_blocks,
 
     cudaStream_t st = (cudaStream_t)stream;
     const int threads = std::max(std::max(P.n, P.grid + 1), F);
-    noalloc_tables_kernel<<<(threads + 255) / 256, 256, 0, st>>>(P);
-    CHX_CUDA(cudaGetLastError());
+    CHX_CUDA(launch_pdl(noalloc_tables_kernel, dim3((threads + 255) / 256), dim3(256), 0, st, P));
     if (P.chunks > 1 && !accumulate)
         CHX_CUDA(cudaMemsetAsync(d_blocks, 0, (size_t)F * P.nb * 2048 * 4, st));
 

@@ -165,10 +165,12 @@ correlate_simt_kernel(const uint8_t *__restrict__ packed, int32_t *__restrict__ 
         }
 }
 
-// Zeroes words of 16 bytes.  The next kernel may start meanwhile (programmatic
-// dependent launch) and waits before it adds to them.
+// Zeroes words of 16 bytes.  The next kernel may start meanwhile, but not before
+// all work ahead of this kernel has ended: it may read its inputs at once and
+// waits only before it writes to the zeroed words.
 __global__ void zero_kernel(uint4 *out, int64_t n) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_wait();
+    pdl_launch_dependents();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x)
         out[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -199,8 +201,10 @@ constexpr int kOaMinGroups = 8;  // groups per CTA below which fewer CTAs are la
 
 __global__ void __launch_bounds__(kOaWarps * 32, 1)
 offset_accumulate_kernel(const uint8_t *__restrict__ packed, uint32_t *__restrict__ sums,
-                         int64_t nvec, int T, int64_t ngroups, int64_t nwork) {
+                         int64_t nvec, int T, int64_t ngroups, int64_t nwork, int zeroed) {
     __shared__ uint32_t part[kOaWarps / 2][32][32];  // [warp pair][word][lane]
+    if (!zeroed) pdl_wait();
+    pdl_launch_dependents();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint4 *p = reinterpret_cast<const uint4 *>(packed);
     const int64_t L1 = nwork * (blockIdx.x + 1) / gridDim.x;
@@ -264,7 +268,7 @@ offset_accumulate_kernel(const uint8_t *__restrict__ packed, uint32_t *__restric
                 part[w - kOaWarps / 2][2 * k + 1][lane] += lo[k];
             }
         __syncthreads();
-        asm volatile("griddepcontrol.wait;" ::: "memory");  // the sums have been zeroed
+        pdl_wait();  // the sums have been zeroed
         // Thread r handles (word, lane) pairs r, r + 512: sum over the warps.
 #pragma unroll
         for (int r = threadIdx.x; r < 32 * 32; r += kOaWarps * 32) {
@@ -326,6 +330,8 @@ __global__ void __launch_bounds__(256)
 preseed_kernel(const uint32_t *__restrict__ sums, int32_t *__restrict__ blocks, int E,
                int nb1, int64_t nb, uint32_t t128, int packed_variant, int ut) {
     __shared__ uint32_t sx[kPsBlocks][64], sy[kPsBlocks][64];
+    pdl_launch_dependents();
+    pdl_wait();
     const int f = blockIdx.y;
     const int64_t b0 = (int64_t)blockIdx.x * kPsBlocks;
     const int tid = threadIdx.x;
@@ -361,6 +367,8 @@ __global__ void __launch_bounds__(256)
 blocks_to_triangle_kernel(const int32_t *__restrict__ blocks, int32_t *__restrict__ tri,
                           int E, int nb1, int64_t nb) {
     __shared__ __align__(16) int2 cells[kTriBlocks][32 * 32];
+    pdl_launch_dependents();
+    pdl_wait();
     const int b0 = blockIdx.x * kTriBlocks, f = blockIdx.y;
     const int n = (int)min((int64_t)kTriBlocks, nb - b0);
     const int64_t ntri = (int64_t)E * (E + 1) / 2;
@@ -407,6 +415,8 @@ __global__ void __launch_bounds__(256)
 blocks_to_full_kernel(const int32_t *__restrict__ blocks, int32_t *__restrict__ full,
                       int E, int nb1, int64_t nb) {
     __shared__ int2 tile[32][33];
+    pdl_launch_dependents();
+    pdl_wait();
     const int b = blockIdx.x, f = blockIdx.y;
     int by, bx;
     decode_block(b, nb1, by, bx);
@@ -464,51 +474,36 @@ cudaError_t launch_offset_accumulate(const uint8_t *packed, uint32_t *sums, int 
     if (cudaGetDevice(&dev) == cudaSuccess)
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(sms, nwork / kOaMinGroups));
-    // zeroed: the previous kernel of the stream is the one zeroing the sums; this
-    // one starts with it.  Otherwise an ordinary launch.
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kOaWarps * 32);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = zeroed ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, offset_accumulate_kernel, packed, sums, nvec, T,
-                                       ngroups, nwork);
-    if (e != cudaSuccess) return e;
-    return cudaGetLastError();
+    return launch_pdl(offset_accumulate_kernel, dim3((unsigned)grid), dim3(kOaWarps * 32), 0, st,
+                      packed, sums, nvec, T, ngroups, nwork, zeroed ? 1 : 0);
 }
 
 cudaError_t launch_zero(void *out, int64_t bytes, cudaStream_t st) {
     const int64_t n = bytes / 16;
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(1184, (n + 1023) / 1024));
-    zero_kernel<<<grid, 256, 0, st>>>(static_cast<uint4 *>(out), n);
-    return cudaGetLastError();
+    return launch_pdl(zero_kernel, dim3(grid), dim3(256), 0, st, static_cast<uint4 *>(out), n);
 }
 
 cudaError_t launch_preseed(const uint32_t *sums, int32_t *blocks, int E, int F, int T,
                            int packed_variant, int ut, cudaStream_t st) {
     const int64_t nb = num_blocks_of(E);
     dim3 grid((unsigned)((nb + kPsBlocks - 1) / kPsBlocks), (unsigned)F);
-    preseed_kernel<<<grid, 256, 0, st>>>(sums, blocks, E, E / 32, nb, (uint32_t)T * 128u,
-                                         packed_variant, ut);
-    return cudaGetLastError();
+    return launch_pdl(preseed_kernel, grid, dim3(256), 0, st, sums, blocks, E, E / 32, nb,
+                      (uint32_t)T * 128u, packed_variant, ut);
 }
 
 cudaError_t launch_blocks_to_triangle(const int32_t *blocks, int32_t *tri, int E, int F,
                                       cudaStream_t st) {
     dim3 grid((unsigned)((num_blocks_of(E) + kTriBlocks - 1) / kTriBlocks), (unsigned)F);
-    blocks_to_triangle_kernel<<<grid, 256, 0, st>>>(blocks, tri, E, E / 32, num_blocks_of(E));
-    return cudaGetLastError();
+    return launch_pdl(blocks_to_triangle_kernel, grid, dim3(256), 0, st, blocks, tri, E, E / 32,
+                      num_blocks_of(E));
 }
 
 cudaError_t launch_blocks_to_full(const int32_t *blocks, int32_t *full, int E, int F,
                                   cudaStream_t st) {
     dim3 grid((unsigned)num_blocks_of(E), (unsigned)F);
-    blocks_to_full_kernel<<<grid, 256, 0, st>>>(blocks, full, E, E / 32, num_blocks_of(E));
-    return cudaGetLastError();
+    return launch_pdl(blocks_to_full_kernel, grid, dim3(256), 0, st, blocks, full, E, E / 32,
+                      num_blocks_of(E));
 }
 
 }  // namespace chx

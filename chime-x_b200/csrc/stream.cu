@@ -77,6 +77,8 @@ struct FrameCopy {
 // All frame copies of one submit in one launch: block y = copy, blocks x
 // stride over its 16-byte words.
 __global__ void frame_copy_kernel(const FrameCopy *copies) {
+    pdl_launch_dependents();
+    pdl_wait();
     const FrameCopy c = copies[blockIdx.y];
     const int64_t words = c.bytes >> 4;
     const uint4 *src = reinterpret_cast<const uint4 *>(c.src);
@@ -89,8 +91,7 @@ __global__ void frame_copy_kernel(const FrameCopy *copies) {
 cudaError_t launch_frame_copies(const FrameCopy *d_copies, int n, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     if (n > 65535) return cudaErrorInvalidValue;
-    frame_copy_kernel<<<dim3(8, n), 256, 0, st>>>(d_copies);
-    return cudaGetLastError();
+    return launch_pdl(frame_copy_kernel, dim3(8, n), dim3(256), 0, st, d_copies);
 }
 
 // The integrations one launch completes, and the event recorded after it.

@@ -99,16 +99,6 @@ static __device__ __noinline__ bool mbar_wait_drain(uint32_t bar, uint32_t parit
         if (globaltimer() - t0 > kWaitLimitNs) return false;
     return true;
 }
-// Programmatic dependent launch.  The next kernel of the stream may start its
-// set-up once every CTA of this one has started; pdl_wait returns when the
-// previous kernel has completed and its writes are visible (at once when the
-// launch did not ask for overlap).
-__device__ __forceinline__ void pdl_launch_dependents() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-__device__ __forceinline__ void pdl_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
 // One lane of a converged warp (the same one each time).
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t p;

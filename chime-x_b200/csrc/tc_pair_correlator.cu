@@ -139,6 +139,7 @@ struct KParams {
     int ut;
     int accumulate;
     int static_tables;  // the tables were complete before the launch
+    int after_zero;     // the previous launch is the one zeroing the output
     uint32_t yscale;  // y rows are scaled by 2^yscale
     int *err;
 };
@@ -219,7 +220,9 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();
-    pdl_wait();
+    // The zeroing kernel started after all earlier work had ended: only the
+    // output waits for it.
+    if (!P.after_zero || warp >= kEpiWarp0) pdl_wait();
 
     if (warp == kProducerWarp) {
         // ------------------------------------------------- TMA producer (both CTAs)
@@ -553,6 +556,7 @@ cudaError_t launch_pair_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t 
     P.ut = L.ut;
     P.accumulate = L.accumulate;
     P.static_tables = L.static_tables;
+    P.after_zero = L.after_zero;
     P.yscale = L.max_samples <= kScaledMaxSamples ? 3 : 0;
     P.err = L.err;
     TcMaps none;

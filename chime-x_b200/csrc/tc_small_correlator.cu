@@ -76,6 +76,7 @@ struct KParams {
     const int *cta_offsets;  // CTA b takes units [cta_offsets[b], cta_offsets[b+1])
     int use_param_map;
     int static_tables;  // the tables were complete before the launch
+    int after_zero;     // the previous launch is the one zeroing the output
     int ut;
     int accumulate;
     int *err;
@@ -173,7 +174,9 @@ tc_small_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant_
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_launch_dependents();
-    pdl_wait();
+    // The zeroing kernel started after all earlier work had ended: only the
+    // output waits for it.
+    if (!P.after_zero || warp >= kEpiWarp0) pdl_wait();
 
     // Stages of a unit, the same for the whole warp.
     auto stages = [&](int u) {
@@ -427,25 +430,15 @@ cudaError_t launch_small_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t
     P.cta_offsets = L.cta_offsets;
     P.use_param_map = L.use_param_map;
     P.static_tables = L.static_tables;
+    P.after_zero = L.after_zero;
     P.ut = L.ut;
     P.accumulate = L.accumulate;
     P.err = L.err;
     TcMaps none;
     memset(&none, 0, sizeof(none));
     const TcMaps &m = maps ? *maps : none;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(L.grid);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmemBytes;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, tc_small_kernel<MAP>, m.in, m.out, P);
-    if (e != cudaSuccess) return e;
-    return cudaGetLastError();
+    return launch_pdl(tc_small_kernel<MAP>, dim3(L.grid), dim3(kThreads), kSmemBytes, st, m.in, m.out,
+                      P);
 }
 
 }  // namespace
