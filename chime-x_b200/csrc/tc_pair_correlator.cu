@@ -355,17 +355,22 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
         const uint32_t yst0 = (uint32_t)gw * 1024 + swz(yr, lane & 7);
         const uint32_t yst1 = (uint32_t)gw * 1024 + swz(yr + 4, lane & 7);
         const uint32_t xst = (uint32_t)gw * 512 + swz64(xr, lane & 3);
-        const uint32_t full_op_leader = mapa(bar(kBarFullOp), 0);
+        // The n-th step of this group is step kGroups n + grp: always operand slot
+        // grp, and packed slots grp and grp + kGroups in turn.
+        static_assert(kOpSlots == kGroups && kPkSlots == 2 * kGroups, "slots of a group");
+        const uint32_t full_op = bar(kBarFullOp + grp), empty_op = bar(kBarEmptyOp + grp);
+        const uint32_t full_op_leader = mapa(full_op, 0);
+        const uint32_t ya0 = op_y + grp * kYOpBytes + yst0, ya1 = op_y + grp * kYOpBytes + yst1;
+        const uint32_t xa = op_x + grp * 2 * kXOpBytes + xst;
         const YScale ys(P.yscale);
-        uint32_t g = 0;  // steps of the units before this one
+        uint32_t n = 0, g = 0;  // this group's steps, all steps of the units before this one
         bool ok = true;
         for (int u = first; u < last && ok; u++) {
             const Unit U = P.units[u];
             const Steps S(U);
-            for (int k = (int)(((uint32_t)grp - g) % kGroups); k < S.total; k += kGroups) {
-                const uint32_t gs = g + (uint32_t)k;
-                const uint32_t ps = gs % kPkSlots;
-                ok = mbar_wait_warp(bar(kBarFullPk) + 8 * ps, (gs / kPkSlots) & 1, abort_flag);
+            for (int k = (int)(((uint32_t)grp - g) % kGroups); k < S.total; k += kGroups, n++) {
+                const uint32_t ps = grp + kGroups * (n & 1);
+                ok = mbar_wait_warp(bar(kBarFullPk) + 8 * ps, (n >> 1) & 1, abort_flag);
                 if (!ok) break;
                 const bool act[2] = {S.lane0(k), S.lane1(k)};
                 uint4 wy[2], wx[2];
@@ -383,7 +388,7 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         yconv_scaled<MAP>(ys, a[q], y[j][0][q], y[j][1][q], y[j][2][q]);
-                        xconv<MAP>(b[q], x[j][0][q], x[j][1][q]);
+                        if (act[j]) xconv<MAP>(b[q], x[j][0][q], x[j][1][q]);
                     }
                 }
                 // One arrival per warp frees the slot.  It must not overtake the
@@ -404,13 +409,11 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
                         }
                     }
                 }
-                const uint32_t os = gs % kOpSlots;
-                ok = mbar_wait_warp(bar(kBarEmptyOp) + 8 * os, ((gs / kOpSlots) & 1) ^ 1, abort_flag);
+                ok = mbar_wait_warp(empty_op, (n & 1) ^ 1, abort_flag);
                 if (!ok) break;
-                const uint32_t ya = op_y + os * kYOpBytes, xa = op_x + os * 2 * kXOpBytes + xst;
 #pragma unroll
                 for (int j = 0; j < 2; j++) {
-                    const uint32_t st = ya + (j ? yst1 : yst0);
+                    const uint32_t st = j ? ya1 : ya0;
 #pragma unroll
                     for (int r = 0; r < 3; r++)
                         sts128(st + r * kYTileBytes, y[j][r][0], y[j][r][1], y[j][r][2], y[j][r][3]);
@@ -427,9 +430,9 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
                 __syncwarp();
                 if (lane == 0) {
                     if (rank == 0)
-                        mbar_arrive(bar(kBarFullOp) + 8 * os);
+                        mbar_arrive(full_op);
                     else
-                        mbar_arrive_cluster(full_op_leader + 8 * os);
+                        mbar_arrive_cluster(full_op_leader);
                 }
             }
             g += (uint32_t)S.total;
