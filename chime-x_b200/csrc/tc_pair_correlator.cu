@@ -141,6 +141,7 @@ struct KParams {
     int static_tables;  // the tables were complete before the launch
     int after_zero;     // the previous launch is the one zeroing the output
     uint32_t yscale;  // y rows are scaled by 2^yscale
+    uint32_t one;  // 1 (YScale)
     int *err;
 };
 
@@ -362,7 +363,7 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
         const uint32_t full_op_leader = mapa(full_op, 0);
         const uint32_t ya0 = op_y + grp * kYOpBytes + yst0, ya1 = op_y + grp * kYOpBytes + yst1;
         const uint32_t xa = op_x + grp * 2 * kXOpBytes + xst;
-        const YScale ys(P.yscale);
+        const YScale ys(P.yscale, P.one);
         uint32_t n = 0, g = 0;  // this group's steps, all steps of the units before this one
         bool ok = true;
         for (int u = first; u < last && ok; u++) {
@@ -561,6 +562,7 @@ cudaError_t launch_pair_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t 
     P.static_tables = L.static_tables;
     P.after_zero = L.after_zero;
     P.yscale = L.max_samples <= kScaledMaxSamples ? 3 : 0;
+    P.one = 1;
     P.err = L.err;
     TcMaps none;
     memset(&none, 0, sizeof(none));

@@ -40,7 +40,7 @@ constexpr int kUnpackWarps = 16;
 constexpr int kGroups = 4;
 constexpr int kGroupWarps = kUnpackWarps / kGroups;
 constexpr int kPkSlots = 10;  // see tc_pair_correlator.cu
-static_assert(kPkSlots >= kGroups + kOpSlots, "parity of the packed ring");
+static_assert(kPkSlots >= kGroups + kOpSlots && kOpSlots >= kGroups, "parity of the rings");
 constexpr int kTileBytes = kStageSamples * 128;
 constexpr int kRowsMax = 4;
 constexpr int kOpBytes = kRowsMax * kTileBytes;
@@ -79,6 +79,7 @@ struct KParams {
     int after_zero;     // the previous launch is the one zeroing the output
     int ut;
     int accumulate;
+    uint32_t one;  // 1 (YScale)
     int *err;
 };
 
@@ -270,7 +271,7 @@ tc_small_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant_
         const uint32_t ld = (uint32_t)(gw * 1024 + lane * 16);
         const uint32_t st0 = (uint32_t)gw * 1024 + swz(r0, chunk);
         const uint32_t st1 = (uint32_t)gw * 1024 + swz(r0 + 4, chunk);
-        const YScale ys(kScale);
+        const YScale ys(kScale, P.one);
         uint32_t g = 0;  // steps of the units before this one
         bool ok = true;
         for (int u = first; u < last && ok; u++) {
@@ -294,7 +295,7 @@ tc_small_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant_
 #pragma unroll
                     for (int q = 0; q < 4; q++) {
                         yconv_scaled<MAP>(ys, b[q], v[j][0][q], v[j][1][q], v[j][2][q]);
-                        v[j][3][q] = (b[q] << ys.shl) & ys.mask;  // x'i (MAP_PACKED)
+                        v[j][3][q] = ys.low(b[q]);  // x'i (MAP_PACKED)
                     }
                 }
                 // The slot's release must not overtake the loads of any lane: the
@@ -433,6 +434,7 @@ cudaError_t launch_small_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t
     P.after_zero = L.after_zero;
     P.ut = L.ut;
     P.accumulate = L.accumulate;
+    P.one = 1;
     P.err = L.err;
     TcMaps none;
     memset(&none, 0, sizeof(none));
