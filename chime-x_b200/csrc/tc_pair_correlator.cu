@@ -22,8 +22,9 @@
 // step k takes stage k mod nst, lane 0 is active in steps [0, nst), lane 1 in
 // [skew, nst + skew).  Lane 0 drains while lane 1 finishes alone, lane 1 drains
 // while lane 0 of the next unit runs alone.  The price is skew more steps of y
-// conversion per unit, and that a step of one lane takes 450-500 cycles (the latency
-// of the operand ring) for half the work of a 512-cycle step of two.  Measured
+// conversion per unit, and that a step of one lane takes 400-480 cycles (the latency
+// of the operand ring, and shared memory while a drain runs) for half the work of
+// a 512-cycle step of two.  Measured
 // against both lanes in step (E = 2048, F = 37, unsplit; sustained): T = 1024
 // 284 -> 272 us, T = 256 141 -> 130 us, T = 16384 unchanged.  Two full units of
 // half the width, with an accumulator buffer each, were bound by shared memory
@@ -281,21 +282,30 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
             uint32_t s = 0, ph = 0;           // operand slot, its phase
             uint32_t aph0 = 0, aph1 = 0;      // accumulator phases of the lanes
             bool ok = true;
-            // Waits for the operands of the next step.
+            // Waits for the operands of the next step, unless the look ahead
+            // during the one before found them: that look's latency passes behind
+            // the MMAs.  Units of one lane only, whose steps take 400 instead of 425
+            // cycles; at the power cap units of two lanes lose 0.5 % to it.
+            bool look = false, ready = false, ahead = false;
             auto step_ready = [&]() {
-                const bool full = mbar_wait_warp<true>(bar(kBarFullOp) + 8 * s, ph, abort_flag);
+                const bool full =
+                    ready || mbar_wait_warp<true>(bar(kBarFullOp) + 8 * s, ph, abort_flag);
                 tc_fence_after();
+                const uint32_t s1 = (s + 1) % kOpSlots;
+                ahead = look && mbar_test_cluster(bar(kBarFullOp) + 8 * s1, s1 == 0 ? ph ^ 1 : ph);
                 return full;
             };
             // Hands the step's slot back and moves on.
             auto step_done = [&]() {
                 mma_commit_pair(lead, bar(kBarEmptyOp) + 8 * s);
+                ready = look && __all_sync(0xffffffffu, ahead);
                 s = (s + 1) % kOpSlots;
                 ph ^= s == 0 ? 1u : 0u;
             };
             // One loop per phase of the unit, so that no step branches.
             for (int u = first; u < last && ok; u++) {
                 const Steps S(P.units[u]);
+                look = !S.two();
                 ok = mbar_wait_warp<true>(bar(kBarAccEmpty), aph0 ^ 1, abort_flag);  // drained
                 aph0 ^= 1;
                 for (int k = 0; ok && k < S.skew; k++) {
