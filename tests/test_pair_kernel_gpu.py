@@ -89,3 +89,20 @@ def test_noalloc_narrow_and_wide_units(cx, E, F, T):
     cx.correlate_noalloc(torch.from_numpy(packed).cuda(), out, E, F, T)
     cx.noalloc_check()
     np.testing.assert_array_equal(out.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("E,F,T", [(1024, 4, 1912), (1024, 4, 330), (256, 75, 200), (128, 150, 400),
+                                   (96, 149, 70)])
+def test_units_beyond_a_whole_wave(cx, E, F, T):
+    """A few units more than the SMs (or SM pairs) take at once may be cut into
+    pieces that add to their cells; others of the launch store theirs."""
+    packed = orc.generate(T, F, E, 4, 1100 + E + T, no_repeat=1)
+    ref = np.concatenate([orc.correlate_channel(packed, T, F, E, f, 0) for f in range(F)])
+    p = cx.Plan(E, F, T, 256, 0)
+    d = torch.from_numpy(packed).cuda()
+    out = torch.full((p.block_words,), 12345, dtype=torch.int32, device="cuda")
+    p.correlate(d, out)
+    np.testing.assert_array_equal(out.cpu().numpy(), ref)
+    p.correlate(d, out, accumulate=True)
+    p.check_device()
+    np.testing.assert_array_equal(out.cpu().numpy(), (ref.astype(np.int64) * 2).astype(np.int32))
