@@ -290,8 +290,10 @@ tc_correlate_kernel(const __grid_constant__ CUtensorMap pmap,
                 }
                 const bool valid = (U.t0 + it * kStageSamples + sy) < U.t1;
                 uint32_t v0[4], v1[4], v2[4], v3[4];  // y: R, I, N; x: X0, Y0, X1, Y1
+                uint32_t seen;  // some of every loaded vector
                 if (is_y) {
                     const uint4 w = lds128(pk_y + ps * kPkYBytes + ldoff);
+                    seen = w.x;
                     yconv<MAP>(w.x, v0[0], v1[0], v2[0]);
                     yconv<MAP>(w.y, v0[1], v1[1], v2[1]);
                     yconv<MAP>(w.z, v0[2], v1[2], v2[2]);
@@ -302,6 +304,7 @@ tc_correlate_kernel(const __grid_constant__ CUtensorMap pmap,
                     const uint4 w0 = lds128(pk_x + ps * kPkXBytes + ldoff);
                     uint4 w1 = make_uint4(0, 0, 0, 0);
                     if (nx > 1) w1 = lds128(pk_x + ps * kPkXBytes + kPkYBytes + ldoff);
+                    seen = w0.x ^ w1.y;
                     xconv<MAP>(w0.x, v0[0], v1[0]);
                     xconv<MAP>(w0.y, v0[1], v1[1]);
                     xconv<MAP>(w0.z, v0[2], v1[2]);
@@ -315,11 +318,11 @@ tc_correlate_kernel(const __grid_constant__ CUtensorMap pmap,
 #pragma unroll
                     for (int k = 0; k < 4; k++) v0[k] = v1[k] = v2[k] = v3[k] = 0u;
                 }
-                // The converted registers depend on the loaded words, and
-                // __syncwarp orders every lane before lane 0's arrive: one
-                // arrival per warp frees the packed slot.
-                __syncwarp();
-                if (lane == 0) mbar_arrive(empty_pk(ps));
+                // One arrival per warp frees the packed slot.  It must not
+                // overtake the loads of any lane: the arriving lane is picked by a
+                // vote over the loaded words (see tc_pair_correlator.cu).
+                const int who = __any_sync(0xffffffffu, seen == 0x9E3779B9u) ? 1 : 0;
+                if (lane == who) mbar_arrive(empty_pk(ps));
 
                 // operand slot of stage `it`: pair (gp_base + it/2), half it&1
                 const uint32_t gpair = gp_base + (uint32_t)(it >> 1);
