@@ -41,10 +41,8 @@ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 void free_plan_device(chx_plan *p) {
     if (p->d_err) cudaFree(p->d_err);
     if (p->d_chans) cudaFree(p->d_chans);
-    if (p->d_units) cudaFree(p->d_units);
     p->d_err = nullptr;
     p->d_chans = nullptr;
-    p->d_units = nullptr;
 }
 
 // Channel table and work units of the tensor-core kernel for the plan's
@@ -60,48 +58,75 @@ cudaError_t build_tc_tables(chx_plan *p) {
         chans[f].fcoord = f;
         chans[f].orow = (int)((int64_t)f * p->NB * 32);
     }
-    std::vector<Unit> units;
     // Unset options: the tile is the autotuner's cached choice for this shape,
     // if any, else the default; the split comes from the makespan estimate,
     // which sees how many units this plan has (the tuner times a workload that
     // fills the GPU, where splitting only adds hand-offs).
-    int tile = p->tile;
+    int default_tile = p->tile;
     int tuned_tile = 0, tuned_split = 0;
-    if (!tile && tc_tune_lookup(p->device, p->E, p->T, &tuned_tile, &tuned_split))
-        tile = tuned_tile;
-    if (!tile) tile = tc_default_tile(p->E);
-    const TcShape shape =
-        tc_choose_shape(tile, p->tsplit, p->sm_count, p->F * p->NB * 8192,
-                        [&](TcShape s, std::vector<int> &costs) {
-                            tc_append_costs(s, p->E, p->T, p->F, costs);
-                        });
-    tile = shape.tile;
-    for (int f = 0; f < p->F; f++)
-        tc_append_tile_units(tile, units, f, p->E, 0, p->T, shape.split, 0);
-    const int slots = tc_tile_slots(tile, p->sm_count);
-    const int grid = (int)std::min<size_t>(units.size(), (size_t)std::max(1, slots));
-    std::vector<int> offsets;
-    tc_schedule(units, grid, offsets);
+    if (!default_tile && tc_tune_lookup(p->device, p->E, p->T, &tuned_tile, &tuned_split))
+        default_tile = tuned_tile;
+    if (!default_tile) default_tile = tc_default_tile(p->E);
+    const int slots = std::max(1, tc_tile_slots(default_tile, p->sm_count));
+    std::vector<Unit> units[2];
+    std::vector<int> offsets[2];
+    size_t bytes = chans.size() * sizeof(ChanDesc);
+    // Launches that add to their output zero nothing, so cutting units costs
+    // them less, and their table may be another one.
+    TcShape uncut{0, 0, 0};  // the first table's shape if its units are not balanced
+    for (int add = 0; add < 2; add++) {
+        const long long zeroing = add ? 0 : tc_zeroing_cost(p->F * p->NB * 8192);
+        const TcShape shape = tc_choose_shape(default_tile, p->tsplit, p->sm_count, zeroing,
+                                              [&](TcShape s, std::vector<int> &costs) {
+                                                  tc_append_costs(s, p->E, p->T, p->F, costs);
+                                              });
+        auto append_units = [&](int tile, int split) {
+            units[add].clear();
+            for (int f = 0; f < p->F; f++)
+                tc_append_tile_units(tile, units[add], f, p->E, 0, p->T, split, 0);
+        };
+        int tile = default_tile;
+        bool balanced = false;
+        if (!p->tsplit && shape.span > 0) {
+            append_units(tile, 1);
+            balanced = tc_balance(shape, tile, p->E, zeroing, units[add], slots, offsets[add]);
+        }
+        if (!balanced && shape.tile == uncut.tile && shape.split == uncut.split) {
+            units[add].clear();
+            p->tc[add] = p->tc[0];
+            continue;
+        }
+        if (!balanced) {
+            uncut = shape;
+            tile = shape.tile;
+            append_units(tile, shape.split);
+            tc_schedule(units[add], (int)std::min<size_t>(units[add].size(), (size_t)slots),
+                        offsets[add]);
+        }
+        auto &t = p->tc[add];
+        t.first = bytes;
+        t.nunits = (int)units[add].size();
+        t.grid = (int)offsets[add].size() - 1;
+        t.tile = tile;
+        t.max_unit = tc_max_samples(units[add]);
+        t.has_split_units = false;
+        for (const Unit &u : units[add]) t.has_split_units |= (u.split != 0);
+        bytes += units[add].size() * sizeof(Unit) + (offsets[add].size() * sizeof(int) + 31) / 32 * 32;
+    }
+    // One allocation and one copy for all tables.
+    std::vector<char> tables(bytes);
+    memcpy(tables.data(), chans.data(), chans.size() * sizeof(ChanDesc));
+    for (int add = 0; add < 2; add++) {
+        if (units[add].empty()) continue;  // shares the other table
+        char *h = tables.data() + p->tc[add].first;
+        const size_t ubytes = units[add].size() * sizeof(Unit);
+        memcpy(h, units[add].data(), ubytes);
+        memcpy(h + ubytes, offsets[add].data(), offsets[add].size() * sizeof(int));
+    }
     if (p->d_chans) cudaFree(p->d_chans);
-    if (p->d_units) cudaFree(p->d_units);
-    p->d_chans = p->d_units = nullptr;
-    const size_t ubytes = units.size() * sizeof(Unit);
-    cudaError_t e = cudaMalloc(&p->d_chans, chans.size() * sizeof(ChanDesc));
-    if (e == cudaSuccess) e = cudaMalloc(&p->d_units, ubytes + offsets.size() * sizeof(int));
-    if (e == cudaSuccess)
-        e = cudaMemcpy(p->d_chans, chans.data(), chans.size() * sizeof(ChanDesc),
-                       cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(p->d_units, units.data(), ubytes, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy((char *)p->d_units + ubytes, offsets.data(), offsets.size() * sizeof(int),
-                       cudaMemcpyHostToDevice);
-    p->nunits = (int)units.size();
-    p->grid = grid;
-    p->tile_built = tile;
-    p->max_unit = tc_max_samples(units);
-    p->has_split_units = false;
-    for (const Unit &u : units) p->has_split_units |= (u.split != 0);
+    p->d_chans = nullptr;
+    cudaError_t e = cudaMalloc(&p->d_chans, bytes);
+    if (e == cudaSuccess) e = cudaMemcpy(p->d_chans, tables.data(), bytes, cudaMemcpyHostToDevice);
     return e;
 }
 
@@ -121,25 +146,26 @@ int run_tc(chx_plan *p, const uint8_t *d_packed, int32_t *d_blocks, int map, int
     const int r = tc_encode_maps(&maps, d_packed, p->E, p->F, p->T, d_blocks);
     if (r != 0) return fail(CHX_E_CUDA, "cuTensorMapEncodeTiled failed (%d)", r);
     TcLaunch L;
-    if (p->has_split_units && !accumulate) {
+    const auto &t = p->tc[accumulate ? 1 : 0];
+    if (t.has_split_units && !accumulate) {
         CHX_CUDA(launch_zero(d_blocks, chx_plan_block_words(p) * 4, st));
         L.after_zero = 1;
     }
     L.chans = (const ChanDesc *)p->d_chans;
-    L.units = (const Unit *)p->d_units;
-    L.nunits = p->nunits;
-    L.max_samples = p->max_unit;
+    L.units = (const Unit *)((const char *)p->d_chans + t.first);
+    L.nunits = t.nunits;
+    L.max_samples = t.max_unit;
     L.max_elements = p->E;
     L.static_tables = 1;
-    L.cta_offsets = (const int *)((const char *)p->d_units + (size_t)p->nunits * sizeof(Unit));
+    L.cta_offsets = (const int *)(L.units + t.nunits);
     L.out_base = (uint64_t)d_blocks;
     L.use_param_map = 1;
     L.map = map;
     L.ut = p->ut;
     L.accumulate = accumulate;
     L.err = p->d_err;
-    L.grid = p->grid;
-    CHX_CUDA(tc_tile_launch(p->tile_built, L, &maps, st));
+    L.grid = t.grid;
+    CHX_CUDA(tc_tile_launch(t.tile, L, &maps, st));
     return CHX_OK;
 }
 
@@ -190,8 +216,6 @@ int chx_plan_create(chx_plan **plan, int E, int F, int T, int TA, int ut, int ke
     p->tile = 0;
     p->d_err = nullptr;
     p->d_chans = nullptr;
-    p->d_units = nullptr;
-    p->nunits = 0;
     cudaError_t e = cudaDeviceGetAttribute(&p->sm_count, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaMalloc(&p->d_err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(p->d_err, 0, sizeof(int));

@@ -197,7 +197,7 @@ int chx_batch_create(chx_batch **out, int n, const chx_channel_desc *descs, int 
     for (int c = 0; c < n; c++)
         out_bytes += descs[c].num_integrations * num_blocks_of(descs[c].num_elements) * 8192;
     const TcShape shape = tc_choose_shape(
-        b->tile, 0, sm_count, out_bytes, [&](TcShape sh, std::vector<int> &costs) {
+        b->tile, 0, sm_count, tc_zeroing_cost(out_bytes), [&](TcShape sh, std::vector<int> &costs) {
             for (int c = 0; c < n; c++)
                 tc_append_costs(sh, descs[c].num_elements, descs[c].num_timesamples,
                                 descs[c].num_integrations, costs);

@@ -44,13 +44,16 @@ struct chx_plan {
     int tile;     // 0 = auto
     int *d_err;   // device error word (bounded-wait timeouts)
     int sm_count;
-    void *d_chans;  // tensor-core channel table (ChanDesc[F])
-    void *d_units;  // tensor-core work units (Unit[nunits]) then grid + 1 offsets
-    int nunits;
-    int grid;       // persistent CTAs (or CTA pairs) of a tensor-core launch
-    int tile_built; // tile variant the tables were built for
-    int max_unit;   // samples of the longest unit
-    bool has_split_units;  // some output cells receive several units (TMA reduce-add)
+    void *d_chans;  // tensor-core channel table (ChanDesc[F]), then both unit tables
+    // Work units of a launch that overwrites its output (0) or adds to it (1).
+    struct {
+        size_t first;   // bytes from d_chans to Unit[nunits], then grid + 1 offsets
+        int nunits;
+        int grid;       // persistent CTAs (or CTA pairs)
+        int tile;       // tile variant
+        int max_unit;   // samples of the longest unit
+        bool has_split_units;  // some output cells receive several units (TMA reduce-add)
+    } tc[2];
 };
 
 namespace chx {
@@ -243,15 +246,25 @@ void tc_schedule(std::vector<Unit> &u, int grid, std::vector<int> &offsets);
 int tc_max_samples(const std::vector<Unit> &u);
 // Makespan of that assignment, in cycles, from the units' costs (sorted here).
 long long tc_estimate_makespan(std::vector<int> &costs, int grid);
-// A tile variant and a number of sample-range splits.
+// Cycles by which zeroing `out_bytes` of output first delays a launch.
+long long tc_zeroing_cost(int64_t out_bytes);
+// A tile variant, a number of sample-range splits and their makespan (0: not
+// estimated).
 struct TcShape {
     int tile, split;
+    long long span;
 };
 // Shape whose units have the shortest estimated makespan: splits 1-32 (split = 0)
 // or the given one, wide or narrow units for the SM pair.  costs_of appends the
-// unit costs of a shape; out_bytes: the output that a split has to zero first.
-TcShape tc_choose_shape(int tile, int split, int sm_count, int64_t out_bytes,
+// unit costs of a shape; zeroing: cycles that a split costs besides
+// (tc_zeroing_cost of an output that has to be zeroed first).
+TcShape tc_choose_shape(int tile, int split, int sm_count, long long zeroing,
                         const std::function<void(TcShape, std::vector<int> &)> &costs_of);
+// Cuts `units` (a whole launch's, unsplit, of `tile` and E elements) into pieces so
+// that every one of at most `slots` CTAs or clusters gets the same cost, and
+// groups them by CTA (offsets: CTAs + 1), if that beats `best` by 5 %.
+bool tc_balance(const TcShape &best, int tile, int E, long long zeroing, std::vector<Unit> &units,
+                int slots, std::vector<int> &offsets);
 // Appends the unit costs of `count` integrations of E elements and T samples.
 void tc_append_costs(TcShape shape, int E, int T, int count, std::vector<int> &costs);
 // Encodes the TMA map of packed samples: dims {E, channels, samples}.

@@ -58,6 +58,10 @@ namespace {
 using namespace tc;
 
 constexpr int kStageSamples = kUnitStageSamples;
+// Shortest piece that tc_balance cuts: 8, 12 and 16 stages measured the same on
+// long units, and 8 up to 10 % faster on short ones (E = 1024, F = 8, T = 1912 40.9,
+// 41.5, 46.0 us; E = 64, F = 1, T = 16384 6.3, 7.7, 7.6).
+constexpr int kMinPieceStages = 8;
 constexpr int kOpStages = 4;    // operand ring
 constexpr int kPkStages = 6;    // packed-tile ring
 constexpr int kYOpBytes = 16 * 1024;  // 12 KiB of operands; the slots also hold the epilogue staging
@@ -612,6 +616,10 @@ int tc_max_samples(const std::vector<Unit> &u) {
 
 long long tc_estimate_makespan(std::vector<int> &costs, int grid) {
     if (grid < 1) grid = 1;
+    // Equal units, the usual case, need neither sorting nor a heap.
+    bool equal = true;
+    for (int c : costs) equal &= c == costs[0];
+    if (equal) return costs.empty() ? 0 : (long long)((costs.size() + grid - 1) / grid) * costs[0];
     std::sort(costs.begin(), costs.end(), std::greater<int>());
     std::priority_queue<long long, std::vector<long long>, std::greater<long long>> load;
     for (int b = 0; b < grid; b++) load.push(0);
@@ -625,7 +633,9 @@ long long tc_estimate_makespan(std::vector<int> &costs, int grid) {
     return span;
 }
 
-TcShape tc_choose_shape(int tile, int split, int sm_count, int64_t out_bytes,
+long long tc_zeroing_cost(int64_t out_bytes) { return 5500 + out_bytes / 2600; }
+
+TcShape tc_choose_shape(int tile, int split, int sm_count, long long zeroing,
                         const std::function<void(TcShape, std::vector<int> &)> &costs_of) {
     // Every range of samples is a unit of its own, with its drain and pipeline
     // latency (unit_cost), so splitting a channel's samples pays only while it
@@ -639,10 +649,8 @@ TcShape tc_choose_shape(int tile, int split, int sm_count, int64_t out_bytes,
     // Narrow SM-pair units (one x tile) cost more per tile than wide ones, but
     // fill idle SM pairs without zeroing and halve a unit's drain; they are tried
     // while the wide units make less than two waves.
-    const long long zeroing = 5500 + out_bytes / 2600;
     const size_t slots = (size_t)std::max(1, tc_tile_slots(tile, sm_count));
-    TcShape best{tile, split ? split : 1};
-    long long best_span = -1;
+    TcShape best{tile, split ? split : 1, 0};
     size_t last_n = 0;
     // More than eight ranges only for launches that would still leave SMs idle
     // (E = 128, F = 1, T = 16384: 20.6 us with 8, 14.4 with 16).
@@ -651,7 +659,7 @@ TcShape tc_choose_shape(int tile, int split, int sm_count, int64_t out_bytes,
         const int k = split ? split : ks[i];
         if (k > 8 && last_n >= slots) break;
         std::vector<int> costs;
-        costs_of(TcShape{tile, k}, costs);
+        costs_of(TcShape{tile, k, 0}, costs);
         const size_t n = costs.size();
         // Eight or more waves of unsplit units leave at most about an eighth
         // of a wave idle, less than the hand-offs that splitting adds.
@@ -660,20 +668,90 @@ TcShape tc_choose_shape(int tile, int split, int sm_count, int64_t out_bytes,
         if (n == last_n) continue;
         last_n = n;
         for (int narrow = 0; narrow < (tile == kTile2Sm && n < 2 * slots ? 2 : 1); narrow++) {
-            const TcShape shape{narrow ? kTileNarrow : tile, k};
+            TcShape shape{narrow ? kTileNarrow : tile, k, 0};
             if (narrow) {
                 costs.clear();
                 costs_of(shape, costs);
             }
             const int grid = (int)std::min(costs.size(), slots);
-            const long long span = tc_estimate_makespan(costs, grid) + (k > 1 ? zeroing : 0);
-            if (best_span < 0 || span * 100 < best_span * 97) {
-                best_span = span;
-                best = shape;
-            }
+            shape.span = tc_estimate_makespan(costs, grid) + (k > 1 ? zeroing : 0);
+            if (best.span == 0 || shape.span * 100 < best.span * 97) best = shape;
         }
     }
     return best;
+}
+
+bool tc_balance(const TcShape &best, int tile, int E, long long zeroing, std::vector<Unit> &units,
+                int slots, std::vector<int> &offsets) {
+    // Equal ranges fit the number of CTAs only by chance: 16 units of four
+    // ranges leave 10 of 74 SM pairs idle, 90 units are a full wave and a fifth
+    // of one.  Laid end to end and cut wherever a CTA's share ends, at most one
+    // unit per CTA is cut in addition, and every CTA ends at the same time.  The
+    // price is zeroing the output (not for launches that add to it) and one
+    // more drain per cut, which unit_cost knows; 5 % is what the estimate was
+    // seen to err.  Measured on B200 (us, equal ranges or none / balanced; in
+    // brackets: adding to the output): E = 256, F = 16, T = 16384 48.2 / 45.2
+    // (45.7 / 41.5), E = 1024, F = 9, T = 4096 80.3 / 66.3 (73.7 / 59.5), E = 512,
+    // F = 30, T = 2048 47.9 / 42.6 (49.5 / 37.0), E = 256, F = 80, T = 4096 71.9 /
+    // 57.0 (67.1 / 52.2), E = 96, F = 64, T = 4096 18.1 / 16.7 (16.6 / 15.6),
+    // E = 1024, F = 4, T = 1912 unchanged (27.9 / 23.5).
+    if (best.span <= 0 || units.empty() || slots < 1) return false;
+    auto cost = [&](const Unit &u, int t0, int t1) {
+        if (tile == kTile1Sm && E <= 128) return small_unit_cost(t0, t1);
+        return unit_cost(tile != kTile1Sm, t0, t1, u.tyx >> 20);
+    };
+    // Fills the CTAs one after the other up to `limit` cycles each; false if
+    // the units do not fit.
+    std::vector<Unit> out;
+    auto pack = [&](long long limit) {
+        out.clear();
+        offsets.assign(1, 0);
+        long long left = limit;
+        for (const Unit &whole : units) {
+            Unit u = whole;
+            while (u.t0 < u.t1) {
+                const int stages = (u.t1 - u.t0 + kStageSamples - 1) / kStageSamples;
+                int n = stages;
+                if (cost(u, u.t0, u.t1) > left) {
+                    // The most stages that fit, leaving a piece worth its drain.
+                    int lo = 0, hi = stages - kMinPieceStages;
+                    while (lo < hi) {
+                        const int mid = (lo + hi + 1) / 2;
+                        if (cost(u, u.t0, u.t0 + mid * kStageSamples) <= left) lo = mid;
+                        else hi = mid - 1;
+                    }
+                    n = lo;
+                    if (n < kMinPieceStages) {
+                        if (left == limit || (int)offsets.size() >= slots) return false;
+                        offsets.push_back((int)out.size());
+                        left = limit;
+                        continue;
+                    }
+                }
+                Unit piece = u;
+                piece.t1 = std::min(u.t1, u.t0 + n * kStageSamples);
+                piece.cost = cost(piece, piece.t0, piece.t1);
+                piece.split |= piece.t0 != whole.t0 || piece.t1 != whole.t1;
+                out.push_back(piece);
+                left -= piece.cost;
+                u.t0 = piece.t1;
+            }
+        }
+        offsets.push_back((int)out.size());
+        return true;
+    };
+    long long lo = 0, hi = best.span * 95 / 100 - zeroing;
+    for (const Unit &u : units) lo += u.cost;
+    lo /= slots;
+    if (hi < lo || !pack(hi)) return false;
+    while (hi - lo > hi / 256) {
+        const long long mid = (lo + hi) / 2;
+        if (pack(mid)) hi = mid;
+        else lo = mid;
+    }
+    pack(hi);
+    units.swap(out);
+    return true;
 }
 
 void tc_append_costs(TcShape shape, int E, int T, int count, std::vector<int> &costs) {

@@ -61,9 +61,9 @@ extern "C" {
 
 /* Plan options. */
 #define CHX_OPT_ALGO 1      /* one of CHX_ALGO_* */
-#define CHX_OPT_TSPLIT 2    /* number of sample-range splits: 0 auto (the
-                               autotuned value, else the split with the
-                               shortest estimated makespan, so that few
+#define CHX_OPT_TSPLIT 2    /* number of sample-range splits: 0 auto (equal
+                               ranges, or equal shares per SM, whichever has
+                               the shortest estimated makespan, so that few
                                channels still fill the GPU), n >= 1 fixed */
 #define CHX_OPT_TILE 3      /* tensor-core tile variant: 0 auto (the
                                autotuned variant, else the SM pair from
