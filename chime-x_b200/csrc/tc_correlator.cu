@@ -49,6 +49,7 @@
 
 #include <algorithm>
 #include <functional>
+#include <numeric>
 #include <queue>
 
 namespace chx {
@@ -674,6 +675,14 @@ TcShape tc_choose_shape(int tile, int split, int sm_count, long long zeroing,
                 costs_of(shape, costs);
             }
             const int grid = (int)std::min(costs.size(), slots);
+            // No assignment ends before its mean load, and more ranges only add
+            // to that: launches that already fill the SMs need few estimates
+            // (E = 2048, F = 8: 200 us of host time per table without this, 4 with).
+            const long long mean = std::accumulate(costs.begin(), costs.end(), 0LL) / grid;
+            if (best.span != 0 && (mean + (k > 1 ? zeroing : 0)) * 100 >= best.span * 97) {
+                if (k > 1 && n >= 2 * slots) return best;
+                continue;
+            }
             shape.span = tc_estimate_makespan(costs, grid) + (k > 1 ? zeroing : 0);
             if (best.span == 0 || shape.span * 100 < best.span * 97) best = shape;
         }
