@@ -204,7 +204,7 @@ __host__ __device__ inline int unit_cost(bool pair, int t0, int t1, int nx) {
 }
 
 // The same for a channel of one 128-element tile (tc_small_correlator.cu): 400
-// per step, and the drains overlap the next unit's steps.
+// per step (250-430 by elements and rows), and the drains overlap the next unit's steps.
 __host__ __device__ inline int small_unit_cost(int t0, int t1) {
     const int stages = (t1 - t0 + kUnitStageSamples - 1) / kUnitStageSamples;
     return 400 * stages + 2000;

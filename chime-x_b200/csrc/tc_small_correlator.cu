@@ -10,20 +10,30 @@
 // no columns are computed in vain, and lanes whose 16 elements lie outside the
 // channel neither load nor store.
 //
+// Two rows (TWO).  N I is the transpose of -I R, so launches of long units neither
+// store N nor multiply by it: K = I R is accumulated, and the epilogue writes
+// K - K^T, taking the transposed blocks through shared memory.  A step has three
+// MMAs and two thirds of the operand stores and reads; the epilogue reads K twice
+// and meets at two barriers.  Per call (us, three rows / two): E = 128, F = 148,
+// T = 4096 32.1 / 27.3, E = 96, F = 64, T = 4096 16.3 / 14.7, E = 64, F = 148, T = 4096
+// 25.9 / 22.2, E = 96, F = 400, T = 768 (24 steps a unit) 19.6 / 18.8, E = 128,
+// F = 160, T = 768 15.6 / 14.4; but E = 96, F = 400, T = 128 (4 steps) 7.9 / 9.8, where
+// the drain sets the pace.  Chosen per launch: choosing per unit in one kernel lost
+// most of the gain (E = 96, F = 64, T = 4096 16.8).
+//
 // Roles and hand-over are those of the SM-pair kernel (tc_pair_correlator.cu):
 // warps 0-15 unpack in four groups, step s in group s % kGroups; 16 TMA
 // producer; 17 MMA issuer; 18-25 epilogue.  TMEM holds two accumulator buffers, so
 // a unit's drain overlaps the next unit's MMAs.
 //
 // What bounds it: shared memory, whose operand stores and reads take about 400
-// cycles per step at N = 128 (430 measured; the step's four M128 MMAs need 2 N),
-// and at small N the unpack warps' latency (290 cycles at N = 32).  Before, the
-// 1-SM kernel of tc_correlator.cu converted the tile twice (y and x), handed
-// its operands over from a lane == 0 branch and drained with its unpack warps:
-// about 1000 cycles per step.  Per call (us, before / now): E = 96, F = 64,
-// T = 4096 43.1 / 20.6, E = 128, F = 148, T = 4096 72.1 / 33.6, E = 32, F = 148,
-// T = 4096 70.0 / 23.8, E = 64, F = 16, T = 16384 41.9 / 18.5, E = 96, F = 1, T = 64
-// 6.9 / 3.9.
+// cycles per step at N = 128 with three rows (430 measured; the step's four M128
+// MMAs need 2 N) and 290 with two, and at small N the unpack warps' latency.
+// Before, the 1-SM kernel of tc_correlator.cu converted the tile twice (y and x),
+// handed its operands over from a lane == 0 branch and drained with its unpack
+// warps: about 1000 cycles per step.  Per call (us, before / now): E = 96, F = 64,
+// T = 4096 43.1 / 14.7, E = 128, F = 148, T = 4096 72.1 / 27.3, E = 32, F = 148,
+// T = 4096 70.0 / 19.3, E = 96, F = 1, T = 64 6.9 / 3.9.
 #include "tc_common.cuh"
 
 #include <string.h>
@@ -43,7 +53,7 @@ constexpr int kPkSlots = 10;  // see tc_pair_correlator.cu
 static_assert(kPkSlots >= kGroups + kOpSlots && kOpSlots >= kGroups, "parity of the rings");
 constexpr int kTileBytes = kStageSamples * 128;
 constexpr int kRowsMax = 4;
-constexpr int kOpBytes = kRowsMax * kTileBytes;
+constexpr int kOpBytesMax = kRowsMax * kTileBytes;
 constexpr int kProducerWarp = 16;
 constexpr int kMmaWarp = 17;
 constexpr int kEpiWarp0 = 18;
@@ -52,13 +62,22 @@ constexpr int kEpiTiles = 2;
 constexpr int kThreads = (kEpiWarp0 + kEpiWarps) * 32;
 constexpr int kTmemCols = 512;  // two buffers of 128 Re and 128 Im columns
 constexpr uint32_t kScale = 2;  // rows scaled by 2^kScale
+// Longest unit from which a launch multiplies two rows (see the top: gains at 24
+// steps and more for every E, losses at 4, even between).
+constexpr int kTwoRowSamples = 24 * kStageSamples;
 
 constexpr int kOffOp = 0;
-constexpr int kOffPk = kOffOp + kOpSlots * kOpBytes;
+constexpr int kOffPk = kOffOp + kOpSlots * kOpBytesMax;
 constexpr int kOffStage = kOffPk + kPkSlots * kTileBytes;
 constexpr int kOffBars = kOffStage + kEpiWarps * kEpiTiles * 4096;
 constexpr int kSmemBytes = kOffBars + 512 + 1024;
 static_assert(kSmemBytes <= 232448, "shared memory per CTA");
+// Two-row operands leave half of their area to the transposed blocks of K: ten of
+// 32 rows of 33 words (no bank conflicts by rows or by columns).
+constexpr int kOffSwap = kOffOp + kOpSlots * 2 * kTileBytes;
+constexpr int kSwapPitch = 33;
+constexpr int kSwapWords = 32 * kSwapPitch;
+static_assert(kOffSwap + 10 * kSwapWords * 4 <= kOffPk, "transposed blocks");
 
 constexpr int kBarFullPk = 0;
 constexpr int kBarEmptyPk = kBarFullPk + kPkSlots;
@@ -114,6 +133,36 @@ __device__ __forceinline__ void mma_step(uint32_t lead, uint32_t d, uint64_t r, 
         "r"(d), "r"(d + 128), "l"(r), "l"(i), "l"(n), "l"(x), "l"(y), "r"(idesc), "r"(acc)
         : "memory");
 }
+// The same for one operand set of two rows:
+//   Re (d) = R R + I I,   K (d + 128) = I R
+__device__ __forceinline__ void mma_step_self(uint32_t lead, uint32_t d, uint64_t r, uint64_t i,
+                                              uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred q, p, t;\n\t"
+        "setp.ne.b32 q, %0, 0;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "setp.eq.b32 t, 0, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::i8 [%1], %3, %3, %5, p;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::i8.collector::a::fill [%2], %4, %3, %5, p;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::i8.collector::a::lastuse [%1], %4, %4, %5, t;\n\t}" ::"r"(
+            lead),
+        "r"(d), "r"(d + 128), "l"(r), "l"(i), "r"(idesc), "r"(acc)
+        : "memory");
+}
+// Barrier of the epilogue warps; true if every thread passed true.
+__device__ __forceinline__ bool epi_barrier(bool ok) {
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, a;\n\t"
+        "setp.ne.b32 p, %1, 0;\n\t"
+        "barrier.cta.red.and.pred a, 1, %2, p;\n\t"
+        "selp.b32 %0, 1, 0, a;\n\t}"
+        : "=r"(all)
+        : "r"(ok ? 1u : 0u), "n"(kEpiWarps * 32)
+        : "memory");
+    __syncwarp();
+    return all != 0;
+}
 __device__ __forceinline__ void mma_commit_lead(uint32_t lead, uint32_t bar) {
     asm volatile(
         "{\n\t.reg .pred q;\n\t"
@@ -124,11 +173,13 @@ __device__ __forceinline__ void mma_commit_lead(uint32_t lead, uint32_t bar) {
         : "memory");
 }
 
-template <int MAP>
+template <int MAP, bool TWO>
 __global__ void __launch_bounds__(kThreads, 1)
 tc_small_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__ CUtensorMap pomap,
                 const KParams P) {
-    constexpr int kRows = MAP == MAP_PACKED ? 4 : 3;  // R, I, N (and the x imaginary row)
+    static_assert(!TWO || MAP != MAP_PACKED, "two rows need equal y and x rows");
+    constexpr int kRows = TWO ? 2 : MAP == MAP_PACKED ? 4 : 3;  // R, I, N, the x imaginary row
+    constexpr int kOpBytes = kRows * kTileBytes;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -236,8 +287,11 @@ tc_small_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant_
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t so = s * (kOpBytes >> 4);
-                mma_step(lead, tmem_base + 256 * a, dR + so, dI + so, dN + so, dR + so, dY + so,
-                         idesc, k > 0 ? 1u : 0u);
+                if (TWO)
+                    mma_step_self(lead, tmem_base + 256 * a, dR + so, dI + so, idesc, k > 0 ? 1u : 0u);
+                else
+                    mma_step(lead, tmem_base + 256 * a, dR + so, dI + so, dN + so, dR + so, dY + so,
+                             idesc, k > 0 ? 1u : 0u);
                 mma_commit_lead(lead, bar(kBarEmptyOp) + 8 * s);
                 g++;
                 s = s + 1 == kOpSlots ? 0 : s + 1;
@@ -344,6 +398,7 @@ tc_small_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant_
         const int j0 = ((warp - kEpiWarp0) >> 2) * 2;
         const uint32_t stage = sbase + kOffStage + (uint32_t)(warp - kEpiWarp0) * kEpiTiles * 4096u;
         const uint32_t lead = elect_one();
+        uint32_t *swap = reinterpret_cast<uint32_t *>(smem + kOffSwap);
         uint32_t a = 0, aph = 0, nchunk = 0;
         bool ok = true;
         for (int u = first; u < last && ok; u++) {
@@ -355,13 +410,35 @@ tc_small_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant_
             const CUtensorMap *omap = P.use_param_map ? &pomap : &cd->omap;
             const int row0 = cd->orow + (int)(U.out_off >> 6);
             ok = mbar_wait_warp(bar(kBarAccFull) + 8 * a, aph, abort_flag);
+            if (TWO) ok = epi_barrier(ok);  // all go on, or none; the last unit's blocks are read
             if (!ok) break;
             tc_fence_after();
+            if (TWO) {
+                // Im = K - K^T: the blocks of K at or below the diagonal go to
+                // shared memory, row x of the block a column, those of the warps'
+                // own parity.
+#pragma unroll 1
+                for (int c = (warp - kEpiWarp0) >> 2; c <= q && q < nb1; c += 2) {
+                    uint32_t *dst = swap + (q * (q + 1) / 2 + c) * kSwapWords + lane;
+                    const uint32_t taddr =
+                        tmem_base + ((uint32_t)(32 * q) << 16) + 256 * a + 128 + 32 * c;
+#pragma unroll
+                    for (int part = 0; part < 4; part++) {
+                        uint32_t k[8];
+                        tmem_ld8(taddr + 8 * part, k);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < 8; i++) dst[(8 * part + i) * kSwapPitch] = k[i];
+                    }
+                }
+                epi_barrier(true);
+            }
 #pragma unroll 1
             for (int j = j0; j < j0 + 2; j++) {
                 if (q >= nb1 || j >= nb1 || j < q) continue;  // warp-uniform
                 const int b = q * nb1 - q * (q - 1) / 2 + (j - q);
                 const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16) + 256 * a + 32 * j;
+                const uint32_t *kt = swap + (j * (j + 1) / 2 + q) * kSwapWords + lane * kSwapPitch;
 #pragma unroll 1
                 for (int half = 0; half < 2; half++) {
                     // Stage the 32 x 32-word tile (rows = lanes) in two
@@ -377,6 +454,7 @@ tc_small_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant_
                         tmem_wait_ld();
 #pragma unroll
                         for (int c = 0; c < 8; c++) {
+                            if (TWO) im[c] -= kt[16 * half + 8 * part + c];
                             re[c] = (uint32_t)((int32_t)re[c] >> (2 * kScale));
                             im[c] = (uint32_t)((int32_t)im[c] >> (2 * kScale));
                             if (!P.ut) im[c] = 0u - im[c];
@@ -412,7 +490,7 @@ tc_small_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant_
     }
 }
 
-template <int MAP>
+template <int MAP, bool TWO>
 cudaError_t launch_small_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t st) {
     static bool attr_done[64] = {};
     int dev = 0;
@@ -420,7 +498,7 @@ cudaError_t launch_small_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!attr_done[dev]) {
-        e = cudaFuncSetAttribute(tc_small_kernel<MAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(tc_small_kernel<MAP, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kSmemBytes);
         if (e != cudaSuccess) return e;
         attr_done[dev] = true;
@@ -439,7 +517,7 @@ cudaError_t launch_small_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t
     TcMaps none;
     memset(&none, 0, sizeof(none));
     const TcMaps &m = maps ? *maps : none;
-    return launch_pdl(tc_small_kernel<MAP>, dim3(L.grid), dim3(kThreads), kSmemBytes, st, m.in, m.out,
+    return launch_pdl(tc_small_kernel<MAP, TWO>, dim3(L.grid), dim3(kThreads), kSmemBytes, st, m.in, m.out,
                       P);
 }
 
@@ -449,10 +527,15 @@ cudaError_t tc_small_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t 
     if (L.nunits <= 0) return cudaSuccess;
     if (L.grid <= 0) return cudaErrorInvalidValue;
     if (L.use_param_map && !maps) return cudaErrorInvalidValue;
+    const bool two = L.max_samples >= kTwoRowSamples;
     switch (L.map) {
-    case MAP_EXACT: return launch_small_map<MAP_EXACT>(L, maps, st);
-    case MAP_CONF: return launch_small_map<MAP_CONF>(L, maps, st);
-    default: return launch_small_map<MAP_PACKED>(L, maps, st);
+    case MAP_EXACT:
+        return two ? launch_small_map<MAP_EXACT, true>(L, maps, st)
+                   : launch_small_map<MAP_EXACT, false>(L, maps, st);
+    case MAP_CONF:
+        return two ? launch_small_map<MAP_CONF, true>(L, maps, st)
+                   : launch_small_map<MAP_CONF, false>(L, maps, st);
+    default: return launch_small_map<MAP_PACKED, false>(L, maps, st);
     }
 }
 

@@ -103,3 +103,42 @@ def test_captured_launches_overlap_safely(cx, E, F, T, tsplit):
     np.testing.assert_array_equal(out.cpu().numpy(), (3 * ref.astype(np.int64)).astype(np.int32))
     np.testing.assert_array_equal(
         tri.cpu().numpy(), orc.blocks_to_triangle((2 * ref.astype(np.int64)).astype(np.int32), F, E))
+
+
+@pytest.mark.parametrize("E", [32, 64, 96, 128])
+@pytest.mark.parametrize("F,T,tsplit,ut", [
+    (2, 736, 1, 1), (2, 737, 1, 0),     # 23 and 24 stages: below and at the two-row rule
+    (2, 768, 1, 1), (1, 769, 1, 0),     # whole stages, one sample of the next
+    (320, 800, 1, 1), (160, 1600, 2, 0),  # several units per SM, split
+    (150, 1500, 0, 1),                  # balanced pieces, short ones among them
+])
+def test_two_row_units(cx, E, F, T, tsplit, ut):
+    """Units whose imaginary part is K - K^T, storing and adding."""
+    packed = np.random.default_rng(E + F + T).integers(0, 256, T * F * E, dtype=np.uint8)
+    p = cx.Plan(E, F, T, 256, ut)
+    p.set_option(cx.OPT_TSPLIT, tsplit)
+    d = torch.from_numpy(packed).cuda()
+    out = p.correlate(d)
+    p.check_device()
+    got = out.view(F, -1).cpu().numpy()
+    for f in {0, F // 2, F - 1}:
+        chan = np.ascontiguousarray(packed.reshape(T, F, E)[:, f]).reshape(-1)
+        np.testing.assert_array_equal(got[f], orc.correlate_blocks(chan, T, 1, E, ut).reshape(-1))
+    twice = p.correlate(d, out.clone(), accumulate=True)
+    p.check_device()
+    assert torch.equal(twice, out * 2)
+
+
+@pytest.mark.parametrize("E", [32, 96, 128])
+@pytest.mark.parametrize("kb,ut", [(0, 1), (0, 0), (1, 1), (1, 0)])
+def test_two_row_offset_maps(cx, E, kb, ut):
+    """The offset-domain maps at lengths where the first multiplies two rows."""
+    T, F = 1024, 1 if kb else 3
+    packed = orc.generate(T, F, E, 4, 810 + E, no_repeat=1)
+    packed[:E] = 0xFF
+    p = cx.Plan(E, F, T, 256, ut, kb)
+    p.set_option(cx.OPT_TSPLIT, 1)
+    zero = torch.zeros(p.block_words, dtype=torch.int32, device="cuda")
+    out = p.corr_compat(torch.from_numpy(packed).cuda(), zero)
+    p.check_device()
+    np.testing.assert_array_equal(out.cpu().numpy(), orc.corr_partials(packed, T, F, E, kb, ut))
