@@ -117,7 +117,9 @@ cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t 
 // Device side of it: the next kernel of the stream may start its set-up once
 // every CTA of this one has called pdl_launch_dependents; pdl_wait returns when
 // the previous kernel has completed and its writes are visible (at once when the
-// launch did not ask for overlap).
+// launch did not ask for overlap).  What the kernel loads may be written until
+// then, within its own lifetime: such loads have to be coherent ones, so no
+// __ldg and no const __restrict__ parameters in these kernels.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

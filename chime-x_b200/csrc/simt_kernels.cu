@@ -200,8 +200,8 @@ constexpr int kOaMinGroups = 8;  // groups per CTA below which fewer CTAs are la
                                  // F = 5, T = 2968: 17.6 us with 1, 6.3 with 8)
 
 __global__ void __launch_bounds__(kOaWarps * 32, 1)
-offset_accumulate_kernel(const uint8_t *__restrict__ packed, uint32_t *__restrict__ sums,
-                         int64_t nvec, int T, int64_t ngroups, int64_t nwork, int zeroed) {
+offset_accumulate_kernel(const uint8_t *packed, uint32_t *sums, int64_t nvec, int T,
+                         int64_t ngroups, int64_t nwork, int zeroed) {
     __shared__ uint32_t part[kOaWarps / 2][32][32];  // [warp pair][word][lane]
     if (!zeroed) pdl_wait();
     pdl_launch_dependents();
@@ -327,8 +327,8 @@ __device__ __forceinline__ void preseed_block(const uint32_t *sx, const uint32_t
 constexpr int kPsBlocks = 4;
 
 __global__ void __launch_bounds__(256)
-preseed_kernel(const uint32_t *__restrict__ sums, int32_t *__restrict__ blocks, int E,
-               int nb1, int64_t nb, uint32_t t128, int packed_variant, int ut) {
+preseed_kernel(const uint32_t *sums, int32_t *blocks, int E, int nb1, int64_t nb, uint32_t t128,
+               int packed_variant, int ut) {
     __shared__ uint32_t sx[kPsBlocks][64], sy[kPsBlocks][64];
     pdl_launch_dependents();
     pdl_wait();
@@ -364,8 +364,7 @@ preseed_kernel(const uint32_t *__restrict__ sums, int32_t *__restrict__ blocks, 
 constexpr int kTriBlocks = 2;
 
 __global__ void __launch_bounds__(256)
-blocks_to_triangle_kernel(const int32_t *__restrict__ blocks, int32_t *__restrict__ tri,
-                          int E, int nb1, int64_t nb) {
+blocks_to_triangle_kernel(const int32_t *blocks, int32_t *tri, int E, int nb1, int64_t nb) {
     __shared__ __align__(16) int2 cells[kTriBlocks][32 * 32];
     pdl_launch_dependents();
     pdl_wait();
@@ -377,7 +376,7 @@ blocks_to_triangle_kernel(const int32_t *__restrict__ blocks, int32_t *__restric
     int4 v[2 * kTriBlocks];
 #pragma unroll
     for (int k = 0; k < 2 * kTriBlocks; k++)
-        if (k < 2 * n) v[k] = __ldg(blk + threadIdx.x + 256 * k);
+        if (k < 2 * n) v[k] = blk[threadIdx.x + 256 * k];
     int by, bx;
     decode_block(b0, nb1, by, bx);
 #pragma unroll
@@ -412,8 +411,7 @@ blocks_to_triangle_kernel(const int32_t *__restrict__ blocks, int32_t *__restric
 // triangle (conjugates) goes through a shared-memory transpose so that its
 // rows are written contiguously too.
 __global__ void __launch_bounds__(256)
-blocks_to_full_kernel(const int32_t *__restrict__ blocks, int32_t *__restrict__ full,
-                      int E, int nb1, int64_t nb) {
+blocks_to_full_kernel(const int32_t *blocks, int32_t *full, int E, int nb1, int64_t nb) {
     __shared__ int2 tile[32][33];
     pdl_launch_dependents();
     pdl_wait();
@@ -422,13 +420,16 @@ blocks_to_full_kernel(const int32_t *__restrict__ blocks, int32_t *__restrict__ 
     decode_block(b, nb1, by, bx);
     const int32_t *blk = blocks + ((int64_t)f * nb + b) * 2048;
     int32_t *m = full + (int64_t)f * E * E * 2;
+    int2 v[4];  // all loads first: the stores may alias them for the compiler
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        v[k] = *reinterpret_cast<const int2 *>(blk + 2 * (threadIdx.x + 256 * k));
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const int c = threadIdx.x + 256 * k, yl = c >> 5, xl = c & 31;
         const int64_t y = by * 32 + yl, x = bx * 32 + xl;
-        const int2 v = *reinterpret_cast<const int2 *>(blk + 2 * c);
-        tile[yl][xl] = v;
-        if (x >= y) *reinterpret_cast<int2 *>(m + (y * E + x) * 2) = v;
+        tile[yl][xl] = v[k];
+        if (x >= y) *reinterpret_cast<int2 *>(m + (y * E + x) * 2) = v[k];
     }
     __syncthreads();
 #pragma unroll

@@ -75,7 +75,7 @@ struct FrameCopy {
 };
 
 // All frame copies of one submit in one launch: block y = copy, blocks x
-// stride over its 16-byte words.
+// stride over its 16-byte words, four loads of a thread in flight.
 __global__ void frame_copy_kernel(const FrameCopy *copies) {
     pdl_launch_dependents();
     pdl_wait();
@@ -83,9 +83,16 @@ __global__ void frame_copy_kernel(const FrameCopy *copies) {
     const int64_t words = c.bytes >> 4;
     const uint4 *src = reinterpret_cast<const uint4 *>(c.src);
     uint4 *dst = reinterpret_cast<uint4 *>(c.dst);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < words;
-         i += (int64_t)gridDim.x * blockDim.x)
-        dst[i] = __ldg(src + i);
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (; i + 3 * step < words; i += 4 * step) {
+        uint4 v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = src[i + k * step];
+#pragma unroll
+        for (int k = 0; k < 4; k++) dst[i + k * step] = v[k];
+    }
+    for (; i < words; i += step) dst[i] = src[i];
 }
 
 cudaError_t launch_frame_copies(const FrameCopy *d_copies, int n, cudaStream_t st) {
