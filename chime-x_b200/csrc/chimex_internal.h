@@ -115,7 +115,11 @@ cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t 
     return cudaGetLastError();
 }
 // Device side of it: the next kernel of the stream may start its set-up once
-// every CTA of this one has called pdl_launch_dependents; pdl_wait returns when
+// every CTA of this one has called pdl_launch_dependents.  A launch that has
+// started waits on SMs that other streams could use, so kernels whose CTAs live
+// long call it when a CTA has issued its last loads, not at their start (two calls
+// of E = 256, F = 18, T = 65536 on 72 SMs, 856 us: a call of E = 256, F = 16,
+// T = 512 on another stream ended after 220 us, 70 now).  pdl_wait returns when
 // the previous kernel has completed and its writes are visible (at once when the
 // launch did not ask for overlap).  What the kernel loads may be written until
 // then, within its own lifetime: such loads have to be coherent ones, so no

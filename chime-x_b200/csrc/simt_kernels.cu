@@ -204,7 +204,6 @@ offset_accumulate_kernel(const uint8_t *packed, uint32_t *sums, int64_t nvec, in
                          int64_t ngroups, int64_t nwork, int zeroed) {
     __shared__ uint32_t part[kOaWarps / 2][32][32];  // [warp pair][word][lane]
     if (!zeroed) pdl_wait();
-    pdl_launch_dependents();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint4 *p = reinterpret_cast<const uint4 *>(packed);
     const int64_t L1 = nwork * (blockIdx.x + 1) / gridDim.x;
@@ -254,6 +253,7 @@ offset_accumulate_kernel(const uint8_t *packed, uint32_t *sums, int64_t nvec, in
                 }
             }
         }
+        if (end == L1) pdl_launch_dependents();
         if (w < kOaWarps / 2)
 #pragma unroll
             for (int k = 0; k < 16; k++) {

@@ -77,7 +77,6 @@ struct FrameCopy {
 // All frame copies of one submit in one launch: block y = copy, blocks x
 // stride over its 16-byte words, four loads of a thread in flight.
 __global__ void frame_copy_kernel(const FrameCopy *copies) {
-    pdl_launch_dependents();
     pdl_wait();
     const FrameCopy c = copies[blockIdx.y];
     const int64_t words = c.bytes >> 4;
@@ -92,6 +91,7 @@ __global__ void frame_copy_kernel(const FrameCopy *copies) {
 #pragma unroll
         for (int k = 0; k < 4; k++) dst[i + k * step] = v[k];
     }
+    pdl_launch_dependents();
     for (; i < words; i += step) dst[i] = src[i];
 }
 

@@ -221,7 +221,6 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
     cluster_sync();  // barriers of both CTAs initialised, TMEM allocated
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    pdl_launch_dependents();
     // The zeroing kernel started after all earlier work had ended: only the
     // output waits for it.
     if (!P.after_zero || warp >= kEpiWarp0) pdl_wait();
@@ -254,6 +253,7 @@ tc_pair_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant__
                 ph ^= s == 0 ? 1u : 0u;
             }
         }
+        pdl_launch_dependents();  // the last steps and drain are left: enough for a set-up
         if (lead) {
             if (!ok) {
                 atomicOr(P.err, 0x100);

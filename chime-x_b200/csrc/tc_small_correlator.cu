@@ -225,7 +225,6 @@ tc_small_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    pdl_launch_dependents();
     // The zeroing kernel started after all earlier work had ended: only the
     // output waits for it.
     if (!P.after_zero || warp >= kEpiWarp0) pdl_wait();
@@ -256,6 +255,7 @@ tc_small_kernel(const __grid_constant__ CUtensorMap pmap, const __grid_constant_
                 ph ^= s == 0 ? 1u : 0u;
             }
         }
+        pdl_launch_dependents();  // the last steps and drain are left: enough for a set-up
         if (lead) {
             if (!ok) {
                 atomicOr(P.err, 0x10);
