@@ -67,6 +67,7 @@ cudaError_t build_tc_tables(chx_plan *p) {
     if (!default_tile && tc_tune_lookup(p->device, p->E, p->T, &tuned_tile, &tuned_split))
         default_tile = tuned_tile;
     if (!default_tile) default_tile = tc_default_tile(p->E);
+    default_tile = tc_launch_tile(default_tile, p->E);
     const int slots = std::max(1, tc_tile_slots(default_tile, p->sm_count));
     std::vector<Unit> units[2];
     std::vector<int> offsets[2];
@@ -89,7 +90,7 @@ cudaError_t build_tc_tables(chx_plan *p) {
         bool balanced = false;
         if (!p->tsplit && shape.span > 0) {
             append_units(tile, 1);
-            balanced = tc_balance(shape, tile, p->E, zeroing, units[add], slots, offsets[add]);
+            balanced = tc_balance(shape, tile, zeroing, units[add], slots, offsets[add]);
         }
         if (!balanced && shape.tile == uncut.tile && shape.split == uncut.split) {
             units[add].clear();
@@ -155,7 +156,6 @@ int run_tc(chx_plan *p, const uint8_t *d_packed, int32_t *d_blocks, int map, int
     L.units = (const Unit *)((const char *)p->d_chans + t.first);
     L.nunits = t.nunits;
     L.max_samples = t.max_unit;
-    L.max_elements = p->E;
     L.static_tables = 1;
     L.cta_offsets = (const int *)(L.units + t.nunits);
     L.out_base = (uint64_t)d_blocks;

@@ -67,7 +67,7 @@ bool tc_tune_lookup(int device, int E, int T, int *tile, int *split) {
 }  // namespace chx
 
 struct chx_batch {
-    int device = 0, ut = 1, n = 0, tile = 0, grid = 0, nunits = 0, max_unit = 0, max_elements = 0;
+    int device = 0, ut = 1, n = 0, tile = 0, grid = 0, nunits = 0, max_unit = 0;
     std::vector<chx_channel_desc> descs;
     chx::ChanDesc *d_chans = nullptr;
     void *d_units = nullptr;  // units then grid + 1 offsets
@@ -106,7 +106,6 @@ int record_batch(chx_batch *b, cudaStream_t st, int accumulate) {
     L.units = (const Unit *)b->d_units;
     L.nunits = b->nunits;
     L.max_samples = b->max_unit;
-    L.max_elements = b->max_elements;
     L.static_tables = 1;
     L.cta_offsets = (const int *)((const char *)b->d_units + (size_t)b->nunits * sizeof(Unit));
     L.out_base = 0;
@@ -170,14 +169,14 @@ int chx_batch_create(chx_batch **out, int n, const chx_channel_desc *descs, int 
     }
 
     // Tile: the autotuned choice of the costliest channel, else the default.
-    int heaviest = 0;
+    int heaviest = 0, max_elements = 0;
     double heaviest_ops = -1;
     for (int c = 0; c < n; c++) {
         const double E = descs[c].num_elements;
         const double ops = 8.0 * E * (E + 1) / 2 * descs[c].num_timesamples *
                            descs[c].num_integrations;
         b->ops += ops;
-        b->max_elements = std::max(b->max_elements, descs[c].num_elements);
+        max_elements = std::max(max_elements, descs[c].num_elements);
         if (ops > heaviest_ops) {
             heaviest_ops = ops;
             heaviest = c;
@@ -187,6 +186,7 @@ int chx_batch_create(chx_batch **out, int n, const chx_channel_desc *descs, int 
     b->tile = tune_lookup(device, descs[heaviest].num_elements, descs[heaviest].num_timesamples, &tv)
                   ? tv.tile
                   : tc_default_tile(descs[heaviest].num_elements);
+    b->tile = tc_launch_tile(b->tile, max_elements);
 
     // Sample splits: one for every channel, chosen for the whole batch by the
     // makespan estimate (a few long channels are split to fill the GPU, many

@@ -193,27 +193,40 @@ constexpr int kUnitStageSamples = 32;      // samples per pipeline stage of both
 // (E = 2048, T = 256 to 16384); below that the drains show again.
 constexpr int kSkewStages = 12;
 
+// Tensor-core tile variants (CHX_OPT_TILE).
+constexpr int kTile1Sm = 1;  // 128 x 256 elements per CTA
+constexpr int kTile2Sm = 2;  // 256 x 256 elements per CTA pair
+constexpr int kTileMax = kTile2Sm;  // last one that a caller can choose
+constexpr int kTileNarrow = 3;      // SM pair with narrow units (tc_choose_shape)
+constexpr int kTileSmall = 4;       // one SM, for launches of channels of one tile only
+constexpr int kSmallElements = 128;  // the largest of these channels
+__host__ __device__ inline bool tile_is_pair(int tile) {
+    return tile == kTile2Sm || tile == kTileNarrow;
+}
+// The variant by which a launch of `tile` runs when its largest channel has
+// max_elements.  Asked once for the whole launch, before its units are made, so
+// that their costs are those of the kernel that runs them.
+inline int tc_launch_tile(int tile, int max_elements) {
+    return tile == kTile1Sm && max_elements <= kSmallElements ? kTileSmall : tile;
+}
+
 // Scheduling cost of a unit over samples [t0, t1), in cycles as measured with
 // clock64: nx x tiles of 128 elements against one y tile (one SM) or two (SM
 // pair).  SM pair: 512 per step of two lanes, 470 per step of one, at least the
 // lanes' drains of 4,700 each, and 1,500 of pipeline latency.  One SM: its
 // stages convert 1 + nx tiles at 330 cycles each, and every unit pays an
-// accumulator hand-off of about 16 stages.  Plans, batches, streams and the
+// accumulator hand-off of about 16 stages.  Channels of one tile by themselves
+// (tc_small_correlator.cu): 400 per step (250-430 by elements and rows), and the
+// drains overlap the next unit's steps.  Plans, batches, streams and the
 // allocation-free entry point share it so that their schedules agree.
-__host__ __device__ inline int unit_cost(bool pair, int t0, int t1, int nx) {
+__host__ __device__ inline int unit_cost(int tile, int t0, int t1, int nx) {
     const int stages = (t1 - t0 + kUnitStageSamples - 1) / kUnitStageSamples;
-    if (!pair) return (stages + 16) * (nx + 1) * 330;
+    if (tile == kTileSmall) return 400 * stages + 2000;
+    if (tile == kTile1Sm) return (stages + 16) * (nx + 1) * 330;
     const int skew = stages < kSkewStages ? stages : kSkewStages;
     const int steps = nx < 2 ? 470 * stages : 512 * (stages - skew) + 2 * 470 * skew;
     const int drain = 4700 * nx;
     return (steps > drain ? steps : drain) + 1500;
-}
-
-// The same for a channel of one 128-element tile (tc_small_correlator.cu): 400
-// per step (250-430 by elements and rows), and the drains overlap the next unit's steps.
-__host__ __device__ inline int small_unit_cost(int t0, int t1) {
-    const int stages = (t1 - t0 + kUnitStageSamples - 1) / kUnitStageSamples;
-    return 400 * stages + 2000;
 }
 
 // The TMA maps of a launch whose channels share them (TcLaunch::use_param_map).
@@ -230,7 +243,6 @@ struct TcLaunch {
     int max_samples;        // samples of the longest unit
     const int *cta_offsets; // device, grid + 1 entries
     uint64_t out_base;      // added to ChanDesc::out
-    int max_elements;       // elements of the largest channel
     int after_zero = 0;     // 1: launch_zero(blocks) was the stream's previous launch
     int static_tables = 0;  // 1: no work of the stream writes the tables
     int use_param_map;      // 1: every channel uses the kernel-parameter map
@@ -242,9 +254,6 @@ struct TcLaunch {
 };
 
 bool tc_supported(int E, int T);
-// Appends the units of one channel's sample range [t_begin, t_end) to `out`.
-void tc_append_units(std::vector<Unit> &out, int chan, int E, int t_begin, int t_end,
-                     int tsplit, long long out_off);
 // Assigns units to `grid` persistent CTAs (longest first, to the least
 // loaded CTA) and reorders them CTA by CTA; offsets gets grid + 1 entries.
 void tc_schedule(std::vector<Unit> &u, int grid, std::vector<int> &offsets);
@@ -266,11 +275,11 @@ struct TcShape {
 // (tc_zeroing_cost of an output that has to be zeroed first).
 TcShape tc_choose_shape(int tile, int split, int sm_count, long long zeroing,
                         const std::function<void(TcShape, std::vector<int> &)> &costs_of);
-// Cuts `units` (a whole launch's, unsplit, of `tile` and E elements) into pieces so
+// Cuts `units` (a whole launch's, unsplit, of `tile`) into pieces so
 // that every one of at most `slots` CTAs or clusters gets the same cost, and
 // groups them by CTA (offsets: CTAs + 1), if that beats `best` by 5 %.
-bool tc_balance(const TcShape &best, int tile, int E, long long zeroing, std::vector<Unit> &units,
-                int slots, std::vector<int> &offsets);
+bool tc_balance(const TcShape &best, int tile, long long zeroing, std::vector<Unit> &units, int slots,
+                std::vector<int> &offsets);
 // Appends the unit costs of `count` integrations of E elements and T samples.
 void tc_append_costs(TcShape shape, int E, int T, int count, std::vector<int> &costs);
 // Encodes the TMA map of packed samples: dims {E, channels, samples}.
@@ -283,12 +292,10 @@ int tc_encode_map(CUtensorMap *m, const void *base, int E, int channels, int64_t
 // stay below 2^31 (tc_out_rows_ok).
 int tc_encode_out_map(CUtensorMap *m, void *base, int64_t rows);
 inline bool tc_out_rows_ok(int64_t rows) { return rows > 0 && rows < (1LL << 31); }
-// maps: the maps every channel uses when L.use_param_map.  Channels of one
-// 128-element tile only go to tc_small_launch.
+// maps: the maps every channel uses when L.use_param_map.
 cudaError_t tc_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st);
 
 // ---- kernel for channels of at most 128 elements (tc_small_correlator.cu) ----
-constexpr int kSmallElements = 128;
 cudaError_t tc_small_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st);
 
 // ---- 2-SM tensor-core kernel (tc_pair_correlator.cu) ----
@@ -301,11 +308,6 @@ void tc_append_pair_units(std::vector<Unit> &out, bool narrow, int chan, int E, 
                           int t_end, int tsplit, long long out_off);
 cudaError_t tc_pair_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st);
 
-// Tensor-core tile variants (CHX_OPT_TILE).
-constexpr int kTile1Sm = 1;  // 128 x 256 elements per CTA
-constexpr int kTile2Sm = 2;  // 256 x 256 elements per CTA pair
-constexpr int kTileMax = kTile2Sm;  // last one that a caller can choose
-constexpr int kTileNarrow = 3;      // SM pair with narrow units (tc_choose_shape)
 int tc_default_tile(int E);
 // Dispatch by tile variant: units of one channel's sample range, persistent
 // CTAs (or clusters) for `sm_count` SMs, and the launch.

@@ -66,8 +66,7 @@ struct UnitClass {
 
 struct TableParams {
     int E, F, T;
-    int pair;    // 1: SM-pair tile, 0: one-SM tile
-    int narrow;  // SM pair: units of one x tile
+    int tile;    // tile variant
     int nt;      // 128-element tiles per channel
     int chunks;  // sample chunks
     int n;       // units
@@ -80,17 +79,18 @@ struct TableParams {
 // tyx of the k-th unit of one channel among the units of its kind, in the
 // order tc_append_pair_units / tc_append_units enumerate them.
 __device__ int kth_tyx(const TableParams &P, int nx, int k) {
-    if (P.pair) {
+    const bool narrow = P.tile == kTileNarrow;
+    if (tile_is_pair(P.tile)) {
         // Narrow: every x tile from the y pair's first one on.  Wide, one lane:
         // the last x tile of every row, when the tile count is odd; two lanes:
         // the x tile pairs.
-        if (nx == 1 && !P.narrow) return k | ((P.nt - 1) << 10) | (1 << 20);
+        if (nx == 1 && !narrow) return k | ((P.nt - 1) << 10) | (1 << 20);
         int ty2 = 0, n;
-        while (k >= (n = P.narrow ? P.nt - 2 * ty2 : P.nt / 2 - ty2)) {
+        while (k >= (n = narrow ? P.nt - 2 * ty2 : P.nt / 2 - ty2)) {
             k -= n;
             ty2++;
         }
-        return ty2 | ((2 * ty2 + (P.narrow ? k : 2 * k)) << 10) | (nx << 20);
+        return ty2 | ((2 * ty2 + (narrow ? k : 2 * k)) << 10) | (nx << 20);
     }
     for (int ty = 0; ty < P.nt; ty++) {
         const int rem = P.nt - ty;  // x tiles at and right of the diagonal
@@ -141,7 +141,7 @@ __global__ void noalloc_tables_kernel(const TableParams P) {
     u.t1 = min(P.T, u.t0 + kUnitMaxSamples);
     u.out_off = 0;
     u.split = P.chunks > 1 ? 1 : 0;
-    u.cost = P.nt == 1 ? small_unit_cost(u.t0, u.t1) : unit_cost(P.pair != 0, u.t0, u.t1, C.nx);
+    u.cost = unit_cost(P.tile, u.t0, u.t1, C.nx);
     // round robin: sorted unit i is the (i / grid)-th unit of CTA i % grid
     const int b = i % P.grid;
     units[b * per_cta + min(b, extra) + i / P.grid] = u;
@@ -196,13 +196,12 @@ cudaError_t scratch_address(int dev, void **out) {
 
 // The unit classes of a call, in decreasing cost; returns the unit count.
 int64_t unit_classes(int E, int F, int T, int tile, TableParams *P) {
-    const bool pair = tile != kTile1Sm, narrow = tile == kTileNarrow;
+    const bool pair = tile_is_pair(tile), narrow = tile == kTileNarrow;
     const int nt = (E + 127) / 128;
     const int chunks = (T + kUnitMaxSamples - 1) / kUnitMaxSamples;
     P->nt = nt;
     P->chunks = chunks;
-    P->pair = pair ? 1 : 0;
-    P->narrow = narrow ? 1 : 0;
+    P->tile = tile;
     P->nclass = 0;
     int64_t per[2] = {0, 0};  // units with two x tiles (lanes), with one
     const int kinds[2] = {2, 1}, nkinds = 2;
@@ -236,7 +235,7 @@ int64_t unit_classes(int E, int F, int T, int tile, TableParams *P) {
     // decreasing cost (at most four classes: insertion sort, no allocation)
     auto cost = [&](const UnitClass &C) {
         const int t0 = C.chunk0 * kUnitMaxSamples;
-        return unit_cost(pair, t0, std::min(T, t0 + kUnitMaxSamples), C.nx);
+        return unit_cost(tile, t0, std::min(T, t0 + kUnitMaxSamples), C.nx);
     };
     for (int a = 1; a < P->nclass; a++)
         for (int b = a; b > 0 && cost(P->cls[b]) > cost(P->cls[b - 1]); b--) {
@@ -283,7 +282,7 @@ extern "C" int chx_correlate_noalloc(const uint8_t *d_packed, int32_t *d_blocks,
     if (F > kNoAllocMaxChannels)
         return fail(CHX_E_UNSUPPORTED, "no-allocation entry point takes at most %d channels (F=%d)",
                     kNoAllocMaxChannels, F);
-    int tile = tc_default_tile(E);
+    int tile = tc_launch_tile(tc_default_tile(E), E);
     TableParams P;
     P.E = E;
     P.F = F;
@@ -308,7 +307,7 @@ extern "C" int chx_correlate_noalloc(const uint8_t *d_packed, int32_t *d_blocks,
         TableParams N = P;
         const int64_t nnarrow = unit_classes(E, F, T, kTileNarrow, &N);
         auto span = [&](int64_t n, int nx) {
-            return (n + slots - 1) / slots * unit_cost(true, 0, std::min(T, kUnitMaxSamples), nx);
+            return (n + slots - 1) / slots * unit_cost(kTile2Sm, 0, std::min(T, kUnitMaxSamples), nx);
         };
         if (span(nnarrow, 1) * 100 < span(nunits, 2) * 97) {
             tile = kTileNarrow;
@@ -334,7 +333,6 @@ extern "C" int chx_correlate_noalloc(const uint8_t *d_packed, int32_t *d_blocks,
     L.units = reinterpret_cast<const Unit *>(dscr + kOffUnits);
     L.nunits = P.n;
     L.max_samples = std::min(T, kUnitMaxSamples);
-    L.max_elements = E;
     L.cta_offsets = reinterpret_cast<const int *>(dscr + kOffOffsets);
     L.out_base = (uint64_t)d_blocks;
     L.use_param_map = 1;

@@ -294,14 +294,9 @@ int chx_stream_admit(chx_stream *s, int E, int TA, int *channel_id) {
     std::vector<Unit> u0, u1;
     const int cid = (int)s->chans.size();
     // The tile variant the plain path would choose for this E.
-    const bool pair = tc_default_tile(E) == kTile2Sm;
-    if (pair) {
-        tc_append_pair_units(u0, false, cid, E, 0, TA, 1, 0);
-        tc_append_pair_units(u1, false, cid, E, TA, 2 * TA, 1, NB * 2048);
-    } else {
-        tc_append_units(u0, cid, E, 0, TA, 1, 0);
-        tc_append_units(u1, cid, E, TA, 2 * TA, 1, NB * 2048);
-    }
+    const int tile = tc_launch_tile(tc_default_tile(E), E);
+    tc_append_tile_units(tile, u0, cid, E, 0, TA, 1, 0);
+    tc_append_tile_units(tile, u1, cid, E, TA, 2 * TA, 1, NB * 2048);
     const int64_t need = ring_bytes + dump_bytes;
     if (s->budget > 0) {
         if (s->resident + need > s->budget)
@@ -350,7 +345,7 @@ int chx_stream_admit(chx_stream *s, int E, int TA, int *channel_id) {
     CHX_CUDA(cudaMemcpy(s->d_chans + cid, &d, sizeof(ChanDesc), cudaMemcpyHostToDevice));
     c.units[0] = std::move(u0);
     c.units[1] = std::move(u1);
-    c.pair = pair;
+    c.pair = tile_is_pair(tile);
     // Grow the per-launch unit tables to hold every channel completing at
     // once.  Growing waits for all launches that read the old tables.
     size_t total_units = c.units[0].size();
@@ -502,19 +497,17 @@ int chx_stream_submit(chx_stream *s, int n, const int *ids, const uint8_t *const
         L.units = (const Unit *)sl.dev;
         L.nunits = (int)units.size();
         L.max_samples = tc_max_samples(units);
-        L.max_elements = 65536;  // not looked at by the SM pair
         L.cta_offsets = (const int *)((const char *)sl.dev + ub);
         L.grid = grid;
-        e = tc_pair_launch(L, nullptr, st);
+        e = tc_tile_launch(kTile2Sm, L, nullptr, st);
     }
     if (e == cudaSuccess && !units1.empty()) {
         L.units = (const Unit *)((const char *)sl.dev + u1b0);
         L.nunits = (int)units1.size();
         L.max_samples = tc_max_samples(units1);
-        L.max_elements = kSmallElements;  // tc_default_tile: one tile
         L.cta_offsets = (const int *)((const char *)sl.dev + u1b0 + u1b);
         L.grid = grid1;
-        e = tc_launch(L, nullptr, st);
+        e = tc_tile_launch(kTileSmall, L, nullptr, st);
     }
     if (e == cudaSuccess) e = cudaEventRecord(sl.done, st);
     if (e != cudaSuccess) {

@@ -483,52 +483,9 @@ cudaError_t launch_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-}  // namespace
-
-// The SM-pair kernel's 256-element units cover an odd number of 128-element
-// tiles with a half-empty row and column of units, whose missing tile's work
-// is done in vain; the one-SM kernel wastes none but converts two x tiles per
-// y tile on one SM.  Measured on B200 with the automatic split (T = 16384,
-// F = 8, TOPS, SM pair / one SM): E = 1920 2427 / 2024, 1664 1998 / 1775,
-// 1408 2051 / 1953, 1152 1903 / 1611, 896 1514 / 1473, 640 1418 / 1449,
-// 384 953 / 732, and 2048 2741 / 2133.  The SM pair is the default from two
-// tiles up; a single tile (E <= 128) would leave three quarters of its one
-// pair unit empty, so it goes to the one-SM tile.  Both stay available as a
-// tile option and to the autotuner.  A launch of the one-SM tile whose channels
-// all fit one 128-element tile runs tc_small_correlator.cu's kernel.
-int tc_default_tile(int E) {
-    const int nt = (E + 127) / 128;
-    return nt >= 2 ? kTile2Sm : kTile1Sm;
-}
-
-void tc_append_tile_units(int tile, std::vector<Unit> &out, int chan, int E, int t_begin,
-                          int t_end, int tsplit, long long out_off) {
-    if (tile != kTile1Sm)
-        tc_append_pair_units(out, tile == kTileNarrow, chan, E, t_begin, t_end, tsplit, out_off);
-    else
-        tc_append_units(out, chan, E, t_begin, t_end, tsplit, out_off);
-}
-
-int tc_tile_slots(int tile, int sm_count) {
-    return tile == kTile1Sm ? sm_count : sm_count / 2;
-}
-
-cudaError_t tc_tile_launch(int tile, const TcLaunch &L, const TcMaps *maps, cudaStream_t st) {
-    if (tile != kTile1Sm) return tc_pair_launch(L, maps, st);
-    return tc_launch(L, maps, st);
-}
-
-int tc_encode_maps(TcMaps *m, const void *d_packed, int E, int F, int T, void *d_blocks) {
-    int r = tc_encode_map(&m->in, d_packed, E, F, T, E, (int64_t)F * E);
-    if (r == 0) r = tc_encode_map(&m->in_half, d_packed, E, F, T, E, (int64_t)F * E, 64);
-    if (r == 0) r = tc_encode_out_map(&m->out, d_blocks, F * num_blocks_of(E) * 32);
-    return r;
-}
-
-bool tc_supported(int E, int T) { return E >= 32 && E % 32 == 0 && E <= 65536 && T >= 1; }
-
-void tc_append_units(std::vector<Unit> &out, int chan, int E, int t_begin, int t_end, int tsplit,
-                     long long out_off) {
+// Units of one channel's sample range for the one-SM tile's kernels.
+void append_units(std::vector<Unit> &out, int tile, int chan, int E, int t_begin, int t_end,
+                  int tsplit, long long out_off) {
     const int nt = (E + 127) / 128;
     const int span = t_end - t_begin;
     if (span <= 0) return;
@@ -548,12 +505,56 @@ void tc_append_units(std::vector<Unit> &out, int chan, int E, int t_begin, int t
                 u.t1 = std::min(t_end, u.t0 + chunk);
                 u.out_off = out_off;
                 u.split = splits > 1 ? 1 : 0;
-                u.cost = nt == 1 ? small_unit_cost(u.t0, u.t1) : unit_cost(false, u.t0, u.t1, nx);
+                u.cost = unit_cost(tile, u.t0, u.t1, nx);
                 out.push_back(u);
             }
         }
     }
 }
+
+}  // namespace
+
+// The SM-pair kernel's 256-element units cover an odd number of 128-element
+// tiles with a half-empty row and column of units, whose missing tile's work
+// is done in vain; the one-SM kernel wastes none but converts two x tiles per
+// y tile on one SM.  Measured on B200 with the automatic split (T = 16384,
+// F = 8, TOPS, SM pair / one SM): E = 1920 2427 / 2024, 1664 1998 / 1775,
+// 1408 2051 / 1953, 1152 1903 / 1611, 896 1514 / 1473, 640 1418 / 1449,
+// 384 953 / 732, and 2048 2741 / 2133.  The SM pair is the default from two
+// tiles up; a single tile (E <= 128) would leave three quarters of its one
+// pair unit empty, so it goes to the one-SM tile.  Both stay available as a
+// tile option and to the autotuner.  A launch of the one-SM tile whose channels
+// all fit one 128-element tile runs tc_small_correlator.cu's kernel (tc_launch_tile).
+int tc_default_tile(int E) {
+    const int nt = (E + 127) / 128;
+    return nt >= 2 ? kTile2Sm : kTile1Sm;
+}
+
+void tc_append_tile_units(int tile, std::vector<Unit> &out, int chan, int E, int t_begin,
+                          int t_end, int tsplit, long long out_off) {
+    if (tile_is_pair(tile))
+        tc_append_pair_units(out, tile == kTileNarrow, chan, E, t_begin, t_end, tsplit, out_off);
+    else
+        append_units(out, tile, chan, E, t_begin, t_end, tsplit, out_off);
+}
+
+int tc_tile_slots(int tile, int sm_count) {
+    return tile_is_pair(tile) ? sm_count / 2 : sm_count;
+}
+
+cudaError_t tc_tile_launch(int tile, const TcLaunch &L, const TcMaps *maps, cudaStream_t st) {
+    if (tile_is_pair(tile)) return tc_pair_launch(L, maps, st);
+    return tile == kTileSmall ? tc_small_launch(L, maps, st) : tc_launch(L, maps, st);
+}
+
+int tc_encode_maps(TcMaps *m, const void *d_packed, int E, int F, int T, void *d_blocks) {
+    int r = tc_encode_map(&m->in, d_packed, E, F, T, E, (int64_t)F * E);
+    if (r == 0) r = tc_encode_map(&m->in_half, d_packed, E, F, T, E, (int64_t)F * E, 64);
+    if (r == 0) r = tc_encode_out_map(&m->out, d_blocks, F * num_blocks_of(E) * 32);
+    return r;
+}
+
+bool tc_supported(int E, int T) { return E >= 32 && E % 32 == 0 && E <= 65536 && T >= 1; }
 
 void tc_schedule(std::vector<Unit> &u, int grid, std::vector<int> &offsets) {
     // Longest-processing-time-first: hand each unit, largest first, to the
@@ -690,8 +691,8 @@ TcShape tc_choose_shape(int tile, int split, int sm_count, long long zeroing,
     return best;
 }
 
-bool tc_balance(const TcShape &best, int tile, int E, long long zeroing, std::vector<Unit> &units,
-                int slots, std::vector<int> &offsets) {
+bool tc_balance(const TcShape &best, int tile, long long zeroing, std::vector<Unit> &units, int slots,
+                std::vector<int> &offsets) {
     // Equal ranges fit the number of CTAs only by chance: 16 units of four
     // ranges leave 10 of 74 SM pairs idle, 90 units are a full wave and a fifth
     // of one.  Laid end to end and cut wherever a CTA's share ends, at most one
@@ -705,10 +706,7 @@ bool tc_balance(const TcShape &best, int tile, int E, long long zeroing, std::ve
     // 57.0 (67.1 / 52.2), E = 96, F = 64, T = 4096 18.1 / 16.7 (16.6 / 15.6),
     // E = 1024, F = 4, T = 1912 unchanged (27.9 / 23.5).
     if (best.span <= 0 || units.empty() || slots < 1) return false;
-    auto cost = [&](const Unit &u, int t0, int t1) {
-        if (tile == kTile1Sm && E <= 128) return small_unit_cost(t0, t1);
-        return unit_cost(tile != kTile1Sm, t0, t1, u.tyx >> 20);
-    };
+    auto cost = [&](const Unit &u, int t0, int t1) { return unit_cost(tile, t0, t1, u.tyx >> 20); };
     // Fills the CTAs one after the other up to `limit` cycles each; false if
     // the units do not fit.
     std::vector<Unit> out;
@@ -818,7 +816,6 @@ cudaError_t tc_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st) {
     if (L.nunits <= 0) return cudaSuccess;
     if (L.grid <= 0) return cudaErrorInvalidValue;
     if (L.use_param_map && !maps) return cudaErrorInvalidValue;
-    if (L.max_elements <= kSmallElements) return tc_small_launch(L, maps, st);
     switch (L.map) {
     case MAP_EXACT: return launch_map<MAP_EXACT>(L, maps, st);
     case MAP_CONF: return launch_map<MAP_CONF>(L, maps, st);

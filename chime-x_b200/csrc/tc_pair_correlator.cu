@@ -619,7 +619,7 @@ void tc_append_pair_units(std::vector<Unit> &out, bool narrow, int chan, int E, 
                 u.t1 = std::min(t_end, u.t0 + chunk);
                 u.out_off = out_off;
                 u.split = splits > 1 ? 1 : 0;
-                u.cost = unit_cost(true, u.t0, u.t1, nl);
+                u.cost = unit_cost(narrow ? kTileNarrow : kTile2Sm, u.t0, u.t1, nl);
                 out.push_back(u);
             }
 }
