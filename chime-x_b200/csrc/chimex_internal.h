@@ -6,6 +6,7 @@
 #include <nvtx3/nvToolsExt.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <functional>
 #include <string>
 #include <vector>
@@ -228,6 +229,18 @@ __host__ __device__ inline int unit_cost(int tile, int t0, int t1, int nx) {
     const int drain = 4700 * nx;
     return (steps > drain ? steps : drain) + 1500;
 }
+// Its inverse: the most stages whose cost is at most `budget` cycles (0: none).
+// tc_balance asks for it once per piece and trial; a search over unit_cost took
+// half of a plan's table building.
+inline int unit_stages(int tile, long long budget, int nx) {
+    if (tile == kTileSmall) return (int)std::max(0LL, (budget - 2000) / 400);
+    if (tile == kTile1Sm) return (int)std::max(0LL, budget / ((nx + 1) * 330) - 16);
+    const long long steps = budget - 1500;
+    if (steps < 4700 * nx) return 0;
+    if (nx < 2) return (int)(steps / 470);
+    const long long skewed = 2 * 470 * kSkewStages;  // both lanes alone for kSkewStages steps
+    return (int)(steps < skewed ? steps / (2 * 470) : kSkewStages + (steps - skewed) / 512);
+}
 
 // The TMA maps of a launch whose channels share them (TcLaunch::use_param_map).
 struct TcMaps {
@@ -259,7 +272,7 @@ bool tc_supported(int E, int T);
 void tc_schedule(std::vector<Unit> &u, int grid, std::vector<int> &offsets);
 // Samples of the longest unit.
 int tc_max_samples(const std::vector<Unit> &u);
-// Makespan of that assignment, in cycles, from the units' costs (sorted here).
+// Makespan of that assignment, in cycles, from the units' costs (reordered here).
 long long tc_estimate_makespan(std::vector<int> &costs, int grid);
 // Cycles by which zeroing `out_bytes` of output first delays a launch.
 long long tc_zeroing_cost(int64_t out_bytes);

@@ -618,19 +618,27 @@ int tc_max_samples(const std::vector<Unit> &u) {
 
 long long tc_estimate_makespan(std::vector<int> &costs, int grid) {
     if (grid < 1) grid = 1;
-    // Equal units, the usual case, need neither sorting nor a heap.
-    bool equal = true;
-    for (int c : costs) equal &= c == costs[0];
-    if (equal) return costs.empty() ? 0 : (long long)((costs.size() + grid - 1) / grid) * costs[0];
-    std::sort(costs.begin(), costs.end(), std::greater<int>());
-    std::priority_queue<long long, std::vector<long long>, std::greater<long long>> load;
-    for (int b = 0; b < grid; b++) load.push(0);
-    long long span = 0;
-    for (int c : costs) {
-        const long long l = load.top() + c;
-        load.pop();
-        load.push(l);
+    if (costs.empty()) return 0;
+    // The longest units, most of them or all as a rule, go round robin; only the
+    // others need sorting and a heap (min-heap of the loads, ascending at first).
+    const int top = *std::max_element(costs.begin(), costs.end());
+    const auto rest = std::partition(costs.begin(), costs.end(), [&](int c) { return c == top; });
+    const long long longest = rest - costs.begin();
+    std::vector<long long> load(grid, longest / grid * top);
+    for (long long i = 0; i < longest % grid; i++) load[grid - 1 - i] += top;
+    long long span = load[grid - 1];
+    std::sort(rest, costs.end(), std::greater<int>());
+    for (auto c = rest; c != costs.end(); ++c) {
+        const long long l = load[0] + *c;
         span = std::max(span, l);
+        int i = 0;
+        for (int child = 1; child < grid; child = 2 * i + 1) {
+            if (child + 1 < grid && load[child + 1] < load[child]) child++;
+            if (load[child] >= l) break;
+            load[i] = load[child];
+            i = child;
+        }
+        load[i] = l;
     }
     return span;
 }
@@ -706,57 +714,59 @@ bool tc_balance(const TcShape &best, int tile, long long zeroing, std::vector<Un
     // 57.0 (67.1 / 52.2), E = 96, F = 64, T = 4096 18.1 / 16.7 (16.6 / 15.6),
     // E = 1024, F = 4, T = 1912 unchanged (27.9 / 23.5).
     if (best.span <= 0 || units.empty() || slots < 1) return false;
-    auto cost = [&](const Unit &u, int t0, int t1) { return unit_cost(tile, t0, t1, u.tyx >> 20); };
     // Fills the CTAs one after the other up to `limit` cycles each; false if
-    // the units do not fit.
+    // the units do not fit.  Writes the pieces and offsets unless it only tries.
     std::vector<Unit> out;
-    auto pack = [&](long long limit) {
-        out.clear();
-        offsets.assign(1, 0);
+    auto pack = [&](long long limit, bool write) {
         long long left = limit;
+        int ctas = 1;
         for (const Unit &whole : units) {
-            Unit u = whole;
-            while (u.t0 < u.t1) {
-                const int stages = (u.t1 - u.t0 + kStageSamples - 1) / kStageSamples;
-                int n = stages;
-                if (cost(u, u.t0, u.t1) > left) {
+            const int nx = whole.tyx >> 20;
+            int t0 = whole.t0, cost = whole.cost;
+            while (true) {
+                int t1 = whole.t1;
+                if (cost > left) {
                     // The most stages that fit, leaving a piece worth its drain.
-                    int lo = 0, hi = stages - kMinPieceStages;
-                    while (lo < hi) {
-                        const int mid = (lo + hi + 1) / 2;
-                        if (cost(u, u.t0, u.t0 + mid * kStageSamples) <= left) lo = mid;
-                        else hi = mid - 1;
-                    }
-                    n = lo;
+                    const int stages = (t1 - t0 + kStageSamples - 1) / kStageSamples;
+                    const int n = std::min(unit_stages(tile, left, nx), stages - kMinPieceStages);
                     if (n < kMinPieceStages) {
-                        if (left == limit || (int)offsets.size() >= slots) return false;
-                        offsets.push_back((int)out.size());
+                        if (left == limit || ctas >= slots) return false;
+                        ctas++;
+                        if (write) offsets.push_back((int)out.size());
                         left = limit;
                         continue;
                     }
+                    t1 = t0 + n * kStageSamples;
+                    cost = unit_cost(tile, t0, t1, nx);
                 }
-                Unit piece = u;
-                piece.t1 = std::min(u.t1, u.t0 + n * kStageSamples);
-                piece.cost = cost(piece, piece.t0, piece.t1);
-                piece.split |= piece.t0 != whole.t0 || piece.t1 != whole.t1;
-                out.push_back(piece);
-                left -= piece.cost;
-                u.t0 = piece.t1;
+                if (write) {
+                    out.push_back(whole);
+                    out.back().t0 = t0;
+                    out.back().t1 = t1;
+                    out.back().cost = cost;
+                    out.back().split |= t0 != whole.t0 || t1 != whole.t1;
+                }
+                left -= cost;
+                if (t1 == whole.t1) break;
+                t0 = t1;
+                cost = unit_cost(tile, t0, whole.t1, nx);
             }
         }
-        offsets.push_back((int)out.size());
         return true;
     };
     long long lo = 0, hi = best.span * 95 / 100 - zeroing;
     for (const Unit &u : units) lo += u.cost;
     lo /= slots;
-    if (hi < lo || !pack(hi)) return false;
+    if (hi < lo || !pack(hi, false)) return false;
     while (hi - lo > hi / 256) {
         const long long mid = (lo + hi) / 2;
-        if (pack(mid)) hi = mid;
+        if (pack(mid, false)) hi = mid;
         else lo = mid;
     }
-    pack(hi);
+    offsets.assign(1, 0);
+    out.reserve(units.size() + slots);
+    pack(hi, true);
+    offsets.push_back((int)out.size());
     units.swap(out);
     return true;
 }

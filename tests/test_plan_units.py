@@ -32,3 +32,20 @@ def test_one_tile_channel_beside_larger_ones(units, T):
     small = units("costs", ONE_SM, 128, T)
     larger = units("costs", ONE_SM, 256, T)
     assert small == [u for u in larger if u[1] == 1]
+
+
+def test_stages_within_a_budget(units):
+    """unit_stages is the inverse of unit_cost."""
+    assert units("inverse") == []
+
+
+# The most time that a plan's two tables may take, as a multiple of what scheduling its
+# units with one to eight equal ranges takes.  Half way (geometrically) between what a
+# search for every piece's length (2.6, 1.20, 1.21, 1.30) and the tables now (1.08, 0.39,
+# 0.38, 0.42) measured.
+@pytest.mark.parametrize("E,F,T,limit", [
+    (256, 16, 16384, 1.7), (96, 64, 4096, 0.7), (64, 65, 5616, 0.7), (32, 67, 11973, 0.7),
+])
+def test_balancing_is_cheap(units, E, F, T, limit):
+    both, equal = min((units("times", E, F, T)[0] for _ in range(3)), key=lambda t: t[0] / t[1])
+    assert both < limit * equal
