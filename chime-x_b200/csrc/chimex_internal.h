@@ -145,6 +145,27 @@ inline int64_t num_blocks_of(int E) {
 cudaError_t launch_correlate_simt(const uint8_t *packed, int32_t *blocks, int E, int F,
                                   int T, int map, int ut, int mode, int splits,
                                   cudaStream_t st);
+// How the offset sums are split: `ctas` CTAs of `warps` warps take equal shares of
+// vblocks vector blocks (512 (f, e) bytes of every sample) x ngroups groups of 16
+// samples.
+struct OffsetSplit {
+    int warps;
+    int64_t ctas;
+};
+constexpr int kOaWarps = 16;      // warps per SM
+constexpr int kOaShortWarps = 4;  // warps per CTA when T is short
+constexpr int kOaMinGroups = 8;   // groups per CTA below which a vector block is not cut:
+                                  // the cuts' atomic adds cost more than their loads (E = 128,
+                                  // F = 5, T = 2968: 17.6 us with 1, 6.3 with 8)
+inline OffsetSplit offset_split(int64_t vblocks, int64_t ngroups, int sms) {
+    // One CTA per SM streams best while every warp has groups of a vector block to
+    // load.  With fewer groups most warps of it would idle, and its vector blocks, about
+    // 2 us each, follow one another: four CTAs per SM then.
+    const int warps = ngroups < kOaWarps ? kOaShortWarps : kOaWarps;
+    // Vector blocks are independent: they always spread over all CTAs.
+    const int64_t work = std::max(vblocks, vblocks * ngroups / kOaMinGroups);
+    return {warps, std::min<int64_t>((int64_t)sms * (kOaWarps / warps), work)};
+}
 // zeroed: launch_zero(sums) was the stream's previous launch.
 cudaError_t launch_offset_accumulate(const uint8_t *packed, uint32_t *sums, int E, int F,
                                      int T, bool zeroed, cudaStream_t st);

@@ -179,11 +179,12 @@ __global__ void zero_kernel(uint4 *out, int64_t n) {
 // offsetAccumulateElements (offset_accumulator.cl:18-47).  The work is the
 // (vector block, 16-sample group) space: a vector block is 32 consecutive
 // 16-byte vectors of a sample row (16 (f, e) bytes each), a group 16 samples.
-// Each CTA (one of 16 warps per SM) takes an equal, contiguous share of that
-// space, so every SM streams the same number of bytes; inside a share, warp w
-// streams the groups w, w + 16, ... of one vector block at a time (each lane
-// one vector: coalesced 512-byte rows), loading a group's 16 vectors at once
-// so that enough bytes are in flight to keep HBM busy (131 KiB per SM).  Four samples' words are
+// Each CTA (16 warps per SM, in one CTA unless T is short: offset_split) takes an
+// equal, contiguous share of that space, so every SM streams the same number of
+// bytes; inside a share, warp w streams the groups w, w + WARPS, ... of one vector
+// block at a time (each lane one vector: coalesced 512-byte rows), loading a group's
+// 16 vectors at once so that enough bytes are in flight to keep HBM busy (131 KiB
+// per SM).  Four samples' words are
 // transposed so that a word holds four samples of one element, whose byte sum
 // (16 re + im) and low-nibble sum (im) are one dp4a each: three ALU instructions
 // per word and 32-bit sums throughout, where masking and adding nibbles in byte
@@ -193,16 +194,14 @@ __global__ void zero_kernel(uint4 *out, int64_t n) {
 // the zeroing, E = 2048, F = 8, T = 16384 (268 MB) took 53.1 us with three CTAs of
 // 8 warps and byte-lane adds, 48.1 with dp4a and two CTAs, 45.4 with one CTA of
 // 16 warps (5.9 TB/s; the read alone 41 us at the copy rate); half as many bytes
-// in flight or twice as many CTAs measured slower.
-constexpr int kOaWarps = 16;
-constexpr int kOaMinGroups = 8;  // groups per CTA below which fewer CTAs are launched:
-                                 // their atomic adds cost more than their loads (E = 128,
-                                 // F = 5, T = 2968: 17.6 us with 1, 6.3 with 8)
-
-__global__ void __launch_bounds__(kOaWarps * 32, 1)
+// in flight or twice as many CTAs measured slower.  Few samples (us, one CTA per
+// eight groups / now; adding): E = 96, F = 55, T = 2 22.2 / 5.9, E = 2048, F = 8, T = 16
+// 14.7 / 6.0, E = 2048, F = 200, T = 200 22.3 / 18.2, E = 2048, F = 1024, T = 1 55.6 / 28.0, T = 128 82.5 / 56.5.
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, kOaWarps / WARPS)
 offset_accumulate_kernel(const uint8_t *packed, uint32_t *sums, int64_t nvec, int T,
                          int64_t ngroups, int64_t nwork, int zeroed) {
-    __shared__ uint32_t part[kOaWarps / 2][32][32];  // [warp pair][word][lane]
+    __shared__ uint32_t part[WARPS / 2][32][32];  // [warp pair][word][lane]
     if (!zeroed) pdl_wait();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint4 *p = reinterpret_cast<const uint4 *>(packed);
@@ -216,7 +215,7 @@ offset_accumulate_kernel(const uint8_t *packed, uint32_t *sums, int64_t nvec, in
 #pragma unroll
         for (int k = 0; k < 16; k++) tot[k] = lo[k] = 0u;
         if (i < nvec) {
-            for (int64_t g = g0 + w; g < g1; g += kOaWarps) {
+            for (int64_t g = g0 + w; g < g1; g += WARPS) {
                 const int t = (int)(16 * g);
                 const uint4 *row = p + (int64_t)t * nvec + i;
                 uint4 v[16];
@@ -254,29 +253,29 @@ offset_accumulate_kernel(const uint8_t *packed, uint32_t *sums, int64_t nvec, in
             }
         }
         if (end == L1) pdl_launch_dependents();
-        if (w < kOaWarps / 2)
+        if (w < WARPS / 2)
 #pragma unroll
             for (int k = 0; k < 16; k++) {
                 part[w][2 * k][lane] = (tot[k] - lo[k]) >> 4;
                 part[w][2 * k + 1][lane] = lo[k];
             }
         __syncthreads();
-        if (w >= kOaWarps / 2)
+        if (w >= WARPS / 2)
 #pragma unroll
             for (int k = 0; k < 16; k++) {
-                part[w - kOaWarps / 2][2 * k][lane] += (tot[k] - lo[k]) >> 4;
-                part[w - kOaWarps / 2][2 * k + 1][lane] += lo[k];
+                part[w - WARPS / 2][2 * k][lane] += (tot[k] - lo[k]) >> 4;
+                part[w - WARPS / 2][2 * k + 1][lane] += lo[k];
             }
         __syncthreads();
         pdl_wait();  // the sums have been zeroed
-        // Thread r handles (word, lane) pairs r, r + 512: sum over the warps.
+        // Thread r handles (word, lane) pairs r, r + 32 WARPS, ...: sum over the warps.
 #pragma unroll
-        for (int r = threadIdx.x; r < 32 * 32; r += kOaWarps * 32) {
+        for (int r = threadIdx.x; r < 32 * 32; r += WARPS * 32) {
             const int k = r >> 5, l = r & 31;
             const int64_t iv = vb * 32 + l;
             uint32_t acc = 0u;
 #pragma unroll
-            for (int ww = 0; ww < kOaWarps / 2; ww++) acc += part[ww][k][l];
+            for (int ww = 0; ww < WARPS / 2; ww++) acc += part[ww][k][l];
             if (iv < nvec && acc != 0u) atomicAdd(sums + 32 * iv + k, acc);
         }
         __syncthreads();  // part is rewritten for the next vector block
@@ -470,13 +469,16 @@ cudaError_t launch_offset_accumulate(const uint8_t *packed, uint32_t *sums, int 
     const int64_t vblocks = (nvec + 31) / 32;
     const int64_t ngroups = (T + 15) / 16;
     const int64_t nwork = vblocks * ngroups;
-    // At most one CTA per SM, each with an equal share of the work.
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess)
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(sms, nwork / kOaMinGroups));
-    return launch_pdl(offset_accumulate_kernel, dim3((unsigned)grid), dim3(kOaWarps * 32), 0, st,
-                      packed, sums, nvec, T, ngroups, nwork, zeroed ? 1 : 0);
+    const OffsetSplit split = offset_split(vblocks, ngroups, sms);
+    const dim3 grid((unsigned)split.ctas), block(split.warps * 32);
+    if (split.warps == kOaWarps)
+        return launch_pdl(offset_accumulate_kernel<kOaWarps>, grid, block, 0, st, packed, sums, nvec,
+                          T, ngroups, nwork, zeroed ? 1 : 0);
+    return launch_pdl(offset_accumulate_kernel<kOaShortWarps>, grid, block, 0, st, packed, sums, nvec,
+                      T, ngroups, nwork, zeroed ? 1 : 0);
 }
 
 cudaError_t launch_zero(void *out, int64_t bytes, cudaStream_t st) {

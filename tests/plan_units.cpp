@@ -93,11 +93,19 @@ static int times(int E, int F, int T) {
     return 0;
 }
 
+// sums VBLOCKS NGROUPS SMS: warps and CTAs of the offset sums.
+static int sums(int vblocks, int ngroups, int sms) {
+    const OffsetSplit s = offset_split(vblocks, ngroups, sms);
+    printf("%d %lld\n", s.warps, (long long)s.ctas);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     auto arg = [&](int i) { return i < argc ? atoi(argv[i]) : 0; };
     if (argc > 1 && !strcmp(argv[1], "costs")) return costs(arg(2), arg(3), arg(4));
     if (argc > 1 && !strcmp(argv[1], "inverse")) return inverse();
     if (argc > 1 && !strcmp(argv[1], "table")) return table(arg(2), arg(3), arg(4), arg(5));
     if (argc > 1 && !strcmp(argv[1], "times")) return times(arg(2), arg(3), arg(4));
+    if (argc > 1 && !strcmp(argv[1], "sums")) return sums(arg(2), arg(3), arg(4));
     return 2;
 }

@@ -30,3 +30,27 @@ def test_offset_sums(E, F, T):
     np.testing.assert_array_equal(sums.cpu().numpy().view(np.uint32), ref)
     p.offset_accumulate(d, sums, accumulate=True)
     np.testing.assert_array_equal(sums.cpu().numpy().view(np.uint32), 2 * ref)
+
+
+@pytest.mark.parametrize("E,F,T", [
+    (96, 55, 1), (96, 55, 2),                     # less than a group in each vector block
+    (2048, 8, 16), (2048, 8, 17),                 # one group, one sample of the next
+    (2048, 300, 1), (2048, 150, 33),              # more vector blocks than CTAs
+    (544, 3, 240), (544, 3, 241), (2048, 4, 255),  # the most groups in short CTAs, one more
+])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_short_offset_sums(E, F, T, accumulate):
+    """Few samples: CTAs of four warps, whole vector blocks."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import chimex as cx
+    packed = np.random.default_rng(E + F + T).integers(0, 256, T * F * E, dtype=np.uint8)
+    packed[:E * F] = 0xFF
+    ref = orc.offset_accumulate(packed, T, F, E)
+    p = cx.Plan(E, F, T)
+    d = torch.from_numpy(packed).cuda()
+    sums = torch.full((p.sum_words,), 5, dtype=torch.int32, device="cuda")
+    for _ in range(2):
+        p.offset_accumulate(d, sums, accumulate=accumulate)
+    ref = ref * 2 + 5 if accumulate else ref
+    np.testing.assert_array_equal(sums.cpu().numpy().view(np.uint32), ref)

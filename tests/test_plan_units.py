@@ -49,3 +49,15 @@ def test_stages_within_a_budget(units):
 def test_balancing_is_cheap(units, E, F, T, limit):
     both, equal = min((units("times", E, F, T)[0] for _ in range(3)), key=lambda t: t[0] / t[1])
     assert both < limit * equal
+
+
+@pytest.mark.parametrize("vblocks,ngroups", [
+    (1, 1), (11, 1), (32, 1), (137, 2), (148, 7), (4096, 1), (4096, 15), (4096, 16), (1, 10000),
+])
+def test_offset_sums_use_every_sm(units, vblocks, ngroups):
+    """No CTA takes a second vector block while another SM could, and short sums, which
+    give few warps of a CTA anything to load, have the warps of an SM in several CTAs."""
+    sms = 148
+    warps, ctas = units("sums", vblocks, ngroups, sms)[0]
+    assert min(vblocks, sms) <= ctas <= min(sms * 16 // warps, vblocks * ngroups)
+    assert warps <= max(4, ngroups)
