@@ -330,6 +330,17 @@ inline bool tc_out_rows_ok(int64_t rows) { return rows > 0 && rows < (1LL << 31)
 cudaError_t tc_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st);
 
 // ---- kernel for channels of at most 128 elements (tc_small_correlator.cu) ----
+// Whether a launch whose longest unit has max_samples multiplies two operand rows
+// instead of three (tc_small_correlator.cu's top): from 24 steps on.  One unit per
+// SM gains there at every E (us, three rows / two: F = 148, T = 768 E = 32 6.9 / 6.3,
+// E = 96 8.3 / 7.9; pieces of at most 28 steps, E = 64, F = 8, T = 16384 9.7 / 9.2); at 4
+// steps two rows lose, between it is even.  Only the longest unit counts, so launches
+// whose other units are short lose: E = 96, F = 100, T = 1000 adding, cut into pieces of
+// mostly 21 steps and fewer, 8.6 / 9.3; a batch of 1000 x (96, 64) beside one
+// (96, 1024) 14.4 / 18.6.
+inline bool small_two_rows(int max_samples) {
+    return (max_samples + kUnitStageSamples - 1) / kUnitStageSamples >= 24;
+}
 cudaError_t tc_small_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t st);
 
 // ---- 2-SM tensor-core kernel (tc_pair_correlator.cu) ----

@@ -62,9 +62,6 @@ constexpr int kEpiTiles = 2;
 constexpr int kThreads = (kEpiWarp0 + kEpiWarps) * 32;
 constexpr int kTmemCols = 512;  // two buffers of 128 Re and 128 Im columns
 constexpr uint32_t kScale = 2;  // rows scaled by 2^kScale
-// Longest unit from which a launch multiplies two rows (see the top: gains at 24
-// steps and more for every E, losses at 4, even between).
-constexpr int kTwoRowSamples = 24 * kStageSamples;
 
 constexpr int kOffOp = 0;
 constexpr int kOffPk = kOffOp + kOpSlots * kOpBytesMax;
@@ -527,7 +524,7 @@ cudaError_t tc_small_launch(const TcLaunch &L, const TcMaps *maps, cudaStream_t 
     if (L.nunits <= 0) return cudaSuccess;
     if (L.grid <= 0) return cudaErrorInvalidValue;
     if (L.use_param_map && !maps) return cudaErrorInvalidValue;
-    const bool two = L.max_samples >= kTwoRowSamples;
+    const bool two = small_two_rows(L.max_samples);
     switch (L.map) {
     case MAP_EXACT:
         return two ? launch_small_map<MAP_EXACT, true>(L, maps, st)

@@ -100,6 +100,12 @@ static int sums(int vblocks, int ngroups, int sms) {
     return 0;
 }
 
+// rows T: operand rows of a small launch whose longest unit has T samples.
+static int rows(int T) {
+    printf("%d\n", small_two_rows(T) ? 2 : 3);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     auto arg = [&](int i) { return i < argc ? atoi(argv[i]) : 0; };
     if (argc > 1 && !strcmp(argv[1], "costs")) return costs(arg(2), arg(3), arg(4));
@@ -107,5 +113,6 @@ int main(int argc, char **argv) {
     if (argc > 1 && !strcmp(argv[1], "table")) return table(arg(2), arg(3), arg(4), arg(5));
     if (argc > 1 && !strcmp(argv[1], "times")) return times(arg(2), arg(3), arg(4));
     if (argc > 1 && !strcmp(argv[1], "sums")) return sums(arg(2), arg(3), arg(4));
+    if (argc > 1 && !strcmp(argv[1], "rows")) return rows(arg(2));
     return 2;
 }

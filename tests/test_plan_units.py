@@ -61,3 +61,9 @@ def test_offset_sums_use_every_sm(units, vblocks, ngroups):
     warps, ctas = units("sums", vblocks, ngroups, sms)[0]
     assert min(vblocks, sms) <= ctas <= min(sms * 16 // warps, vblocks * ngroups)
     assert warps <= max(4, ngroups)
+
+
+@pytest.mark.parametrize("T,rows", [(1, 3), (736, 3), (737, 2), (767, 2), (768, 2), (769, 2)])
+def test_two_rows_from_24_steps(units, T, rows):
+    """A last step of less than 32 samples counts as one."""
+    assert units("rows", T) == [[rows]]
