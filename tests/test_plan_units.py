@@ -67,3 +67,29 @@ def test_offset_sums_use_every_sm(units, vblocks, ngroups):
 def test_two_rows_from_24_steps(units, T, rows):
     """A last step of less than 32 samples counts as one."""
     assert units("rows", T) == [[rows]]
+
+
+@pytest.mark.parametrize("E,F,T,storing,adding", [
+    (256, 16, 16384, 1, 1), (1024, 9, 4096, 1, 1), (512, 30, 2048, 1, 1), (96, 64, 4096, 1, 1),
+    (64, 1, 16384, 1, 1), (128, 3, 300001, 1, 1),
+    (1024, 4, 1912, 0, 1),                      # zeroing the output would cost more than it gives
+    (2048, 8, 16384, 0, 0), (256, 1, 256, 0, 0),  # whole waves; too short to cut
+])
+def test_which_plans_are_balanced(units, E, F, T, storing, adding):
+    """Automatic plans cut units to equal shares per SM where that is worth it, and each
+    of their tables covers every tile pair of every channel once, with the units of a
+    cut range marked as adding."""
+    for add, balanced in ((0, storing), (1, adding)):
+        table = units("table", E, F, T, add)
+        assert table[0] == [balanced]
+        ranges = {}
+        for chan, tyx, t0, t1, split, _ in table[1:]:
+            ranges.setdefault((chan, tyx), []).append((t0, t1, split))
+        assert len(ranges) % F == 0
+        for r in ranges.values():
+            r.sort()
+            assert r[0][0] == 0 and r[-1][1] == T
+            assert all(a[1] == b[0] for a, b in zip(r, r[1:]))
+            assert all(s == (len(r) > 1) for _, _, s in r)
+        if balanced:  # at most one cut per SM besides those of the longest unit
+            assert len(ranges) < len(table) - 1 <= len(ranges) * -(-T // 262144) + 148
