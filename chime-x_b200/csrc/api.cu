@@ -52,7 +52,6 @@ cudaError_t build_tc_tables(chx_plan *p) {
     std::vector<ChanDesc> chans(p->F);
     memset(chans.data(), 0, chans.size() * sizeof(ChanDesc));
     for (int f = 0; f < p->F; f++) {
-        chans[f].out = (uint64_t)f * (uint64_t)p->NB * 2048u * 4u;
         chans[f].E = p->E;
         chans[f].nb1 = (int)p->NB1;
         chans[f].fcoord = f;
@@ -63,10 +62,8 @@ cudaError_t build_tc_tables(chx_plan *p) {
     // which sees how many units this plan has (the tuner times a workload that
     // fills the GPU, where splitting only adds hand-offs).
     int default_tile = p->tile;
-    int tuned_tile = 0, tuned_split = 0;
-    if (!default_tile && tc_tune_lookup(p->device, p->E, p->T, &tuned_tile, &tuned_split))
-        default_tile = tuned_tile;
-    if (!default_tile) default_tile = tc_default_tile(p->E);
+    if (!default_tile && !tc_tune_lookup(p->device, p->E, p->T, &default_tile))
+        default_tile = tc_default_tile(p->E);
     default_tile = tc_launch_tile(default_tile, p->E);
     const int slots = std::max(1, tc_tile_slots(default_tile, p->sm_count));
     std::vector<Unit> units[2];
@@ -158,7 +155,6 @@ int run_tc(chx_plan *p, const uint8_t *d_packed, int32_t *d_blocks, int map, int
     L.max_samples = t.max_unit;
     L.static_tables = 1;
     L.cta_offsets = (const int *)(L.units + t.nunits);
-    L.out_base = (uint64_t)d_blocks;
     L.use_param_map = 1;
     L.map = map;
     L.ut = p->ut;

@@ -56,11 +56,10 @@ bool tune_lookup(int device, int E, int T, TuneVal *out) {
 
 }  // namespace
 
-bool tc_tune_lookup(int device, int E, int T, int *tile, int *split) {
+bool tc_tune_lookup(int device, int E, int T, int *tile) {
     TuneVal tv;
     if (!tune_lookup(device, E, T, &tv)) return false;
     *tile = tv.tile;
-    *split = tv.split;
     return true;
 }
 
@@ -108,7 +107,6 @@ int record_batch(chx_batch *b, cudaStream_t st, int accumulate) {
     L.max_samples = b->max_unit;
     L.static_tables = 1;
     L.cta_offsets = (const int *)((const char *)b->d_units + (size_t)b->nunits * sizeof(Unit));
-    L.out_base = 0;
     L.use_param_map = 0;
     L.map = MAP_EXACT;
     L.ut = b->ut;
@@ -228,7 +226,6 @@ int chx_batch_create(chx_batch **out, int n, const chx_channel_desc *descs, int 
             return fail(CHX_E_CUDA, "channel %d: cuTensorMapEncodeTiled (blocks) failed (%d)", c, r2);
         }
         chans[c].orow = 0;
-        chans[c].out = (uint64_t)d.d_blocks;
         chans[c].E = d.num_elements;
         chans[c].nb1 = d.num_elements / 32;
         chans[c].fcoord = 0;

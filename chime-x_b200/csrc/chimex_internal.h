@@ -180,18 +180,16 @@ cudaError_t launch_blocks_to_full(const int32_t *blocks, int32_t *full, int E, i
 
 // ---- tensor-core kernel (tc_correlator.cu) ----
 // A channel as the tensor-core kernel sees it: the TMA map of its packed
-// samples (dims {E, channels, samples}), its block-buffer address and shape.
+// samples (dims {E, channels, samples}), that of its block buffer, and its shape.
 struct __align__(64) ChanDesc {
     CUtensorMap map;   // samples (128-element tiles); used unless the launch passes one map for all channels
     CUtensorMap xmap;  // samples in 64-element tiles (x of the SM-pair kernel); same rule
     CUtensorMap omap;  // block output as rows of 64 words (tc_encode_out_map); same rule
-    uint64_t out;      // block buffer: absolute address, or byte offset added to
-                       // the launch's out_base
     int E;             // elements
     int nb1;           // E / 32
     int fcoord;        // channel coordinate inside the TMA map
     int orow;          // first row of this channel's blocks inside omap
-    int pad[10];
+    int pad[12];
 };
 static_assert(sizeof(ChanDesc) == 448, "ChanDesc layout");
 
@@ -208,7 +206,7 @@ struct Unit {
 static_assert(sizeof(Unit) == 32, "Unit layout");
 
 constexpr int kUnitMaxSamples = 1 << 18;  // int32-exact bound per unit
-constexpr int kUnitStageSamples = 32;      // samples per pipeline stage of both kernels
+constexpr int kUnitStageSamples = 32;      // samples per pipeline stage of the kernels
 
 // Steps by which the SM-pair kernel's second x lane trails the first: about
 // one lane's accumulator drain.  8 to 14 measured within 1 % of each other
@@ -276,7 +274,6 @@ struct TcLaunch {
     int nunits;
     int max_samples;        // samples of the longest unit
     const int *cta_offsets; // device, grid + 1 entries
-    uint64_t out_base;      // added to ChanDesc::out
     int after_zero = 0;     // 1: launch_zero(blocks) was the stream's previous launch
     int static_tables = 0;  // 1: no work of the stream writes the tables
     int use_param_map;      // 1: every channel uses the kernel-parameter map
@@ -367,8 +364,7 @@ int tc_encode_maps(TcMaps *m, const void *d_packed, int E, int F, int T, void *d
 // device (noalloc.cu); the bounded-wait self-test writes it in mode 2.
 cudaError_t noalloc_error_word(int **out);
 // The autotuner's cached choice for (device, E, T) (batch.cu): true and the
-// tile variant and split count when an entry with the same E and a T within a
-// factor 2 exists.
-bool tc_tune_lookup(int device, int E, int T, int *tile, int *split);
+// tile variant when an entry with the same E and a T within a factor 2 exists.
+bool tc_tune_lookup(int device, int E, int T, int *tile);
 
 }  // namespace chx

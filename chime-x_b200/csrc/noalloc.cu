@@ -118,7 +118,6 @@ __global__ void noalloc_tables_kernel(const TableParams P) {
         int4 *w = reinterpret_cast<int4 *>(chans + i);
         for (int k = 0; k < (int)(sizeof(ChanDesc) / sizeof(int4)); k++)
             w[k] = make_int4(0, 0, 0, 0);
-        chans[i].out = (uint64_t)i * (uint64_t)P.nb * 2048u * 4u;
         chans[i].E = P.E;
         chans[i].nb1 = P.E / 32;
         chans[i].fcoord = i;
@@ -334,7 +333,6 @@ extern "C" int chx_correlate_noalloc(const uint8_t *d_packed, int32_t *d_blocks,
     L.nunits = P.n;
     L.max_samples = std::min(T, kUnitMaxSamples);
     L.cta_offsets = reinterpret_cast<const int *>(dscr + kOffOffsets);
-    L.out_base = (uint64_t)d_blocks;
     L.use_param_map = 1;
     L.map = MAP_EXACT;
     L.ut = upper_triangle_convention;

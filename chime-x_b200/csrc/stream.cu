@@ -338,7 +338,6 @@ int chx_stream_admit(chx_stream *s, int E, int TA, int *channel_id) {
         return fail(CHX_E_CUDA, "cuTensorMapEncodeTiled (dumps) failed (%d)", r2);
     }
     d.orow = 0;
-    d.out = (uint64_t)c.dumps;
     d.E = E;
     d.nb1 = E / 32;
     d.fcoord = 0;
@@ -487,7 +486,6 @@ int chx_stream_submit(chx_stream *s, int n, const int *ids, const uint8_t *const
                                 st);
     TcLaunch L;
     L.chans = s->d_chans;
-    L.out_base = 0;
     L.use_param_map = 0;
     L.map = MAP_EXACT;
     L.ut = s->ut;

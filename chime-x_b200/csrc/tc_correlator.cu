@@ -89,9 +89,7 @@ static_assert(kUnpackWarps * 8192 <= kOffPkY - kOffOpY, "epilogue staging");
 struct KParams {
     const ChanDesc *chans;
     const Unit *units;
-    int nunits;
     const int *cta_offsets;  // CTA b takes units [cta_offsets[b], cta_offsets[b+1])
-    uint64_t out_base;
     int use_param_map;
     int ut;
     int accumulate;
@@ -469,9 +467,7 @@ cudaError_t launch_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t st) {
     KParams P;
     P.chans = L.chans;
     P.units = L.units;
-    P.nunits = L.nunits;
     P.cta_offsets = L.cta_offsets;
-    P.out_base = L.out_base;
     P.use_param_map = L.use_param_map;
     P.ut = L.ut;
     P.accumulate = L.accumulate;

@@ -135,7 +135,6 @@ struct KParams {
     const ChanDesc *chans;
     const Unit *units;
     const int *cluster_offsets;  // cluster c takes units [off[c], off[c+1])
-    uint64_t out_base;
     int use_param_map;
     int ut;
     int accumulate;
@@ -565,7 +564,6 @@ cudaError_t launch_pair_map(const TcLaunch &L, const TcMaps *maps, cudaStream_t 
     P.chans = L.chans;
     P.units = L.units;
     P.cluster_offsets = L.cta_offsets;
-    P.out_base = L.out_base;
     P.use_param_map = L.use_param_map;
     P.ut = L.ut;
     P.accumulate = L.accumulate;
