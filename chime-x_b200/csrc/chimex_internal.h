@@ -233,16 +233,19 @@ inline int tc_launch_tile(int tile, int max_elements) {
 // Scheduling cost of a unit over samples [t0, t1), in cycles as measured with
 // clock64: nx x tiles of 128 elements against one y tile (one SM) or two (SM
 // pair).  SM pair: 512 per step of two lanes, 470 per step of one, at least the
-// lanes' drains of 4,700 each, and 1,500 of pipeline latency.  One SM: its
-// stages convert 1 + nx tiles at 330 cycles each, and every unit pays an
-// accumulator hand-off of about 16 stages.  Channels of one tile by themselves
+// lanes' drains of 4,700 each, and 1,500 of pipeline latency.  One SM: 910 per stage
+// of two x tiles, but 890 of one (the unpack warps' passes set the pace, not the bytes),
+// and 6,000 for each x tile's accumulator hand-off (one unit per SM, T = 512 / 16384: 18.7
+// / 249.7 us with two x tiles, 14.4 / 242.0 with one, 29.0 / 482.7 one of each).  With 2 : 3
+// for them, cut plans gave some SMs half as much again as others (E = 640, F = 8,
+// T = 16384 169 us, 135 now; E = 1920 977, 900).  Channels of one tile by themselves
 // (tc_small_correlator.cu): 400 per step (250-430 by elements and rows), and the
 // drains overlap the next unit's steps.  Plans, batches, streams and the
 // allocation-free entry point share it so that their schedules agree.
 __host__ __device__ inline int unit_cost(int tile, int t0, int t1, int nx) {
     const int stages = (t1 - t0 + kUnitStageSamples - 1) / kUnitStageSamples;
     if (tile == kTileSmall) return 400 * stages + 2000;
-    if (tile == kTile1Sm) return (stages + 16) * (nx + 1) * 330;
+    if (tile == kTile1Sm) return (870 + 20 * nx) * stages + 6000 * nx;
     const int skew = stages < kSkewStages ? stages : kSkewStages;
     const int steps = nx < 2 ? 470 * stages : 512 * (stages - skew) + 2 * 470 * skew;
     const int drain = 4700 * nx;
@@ -253,7 +256,7 @@ __host__ __device__ inline int unit_cost(int tile, int t0, int t1, int nx) {
 // half of a plan's table building.
 inline int unit_stages(int tile, long long budget, int nx) {
     if (tile == kTileSmall) return (int)std::max(0LL, (budget - 2000) / 400);
-    if (tile == kTile1Sm) return (int)std::max(0LL, budget / ((nx + 1) * 330) - 16);
+    if (tile == kTile1Sm) return (int)std::max(0LL, (budget - 6000 * nx) / (870 + 20 * nx));
     const long long steps = budget - 1500;
     if (steps < 4700 * nx) return 0;
     if (nx < 2) return (int)(steps / 470);

@@ -93,3 +93,17 @@ def test_which_plans_are_balanced(units, E, F, T, storing, adding):
             assert all(s == (len(r) > 1) for _, _, s in r)
         if balanced:  # at most one cut per SM besides those of the longest unit
             assert len(ranges) < len(table) - 1 <= len(ranges) * -(-T // 262144) + 148
+
+
+# us for one unit per SM of two x tiles and of one on the one-SM tile, at 1965 MHz.
+ONE_SM_US = {2: {512: 18.7, 4096: 71.9, 16384: 249.7}, 1: {512: 14.4, 4096: 66.2, 16384: 242.0}}
+
+
+@pytest.mark.parametrize("nx", [1, 2])
+@pytest.mark.parametrize("T", [4096, 16384])
+def test_one_sm_unit_costs_follow_the_measured_times(units, nx, T):
+    """Cycles between two lengths, within 5 %, what a balanced plan has to gain at least.
+    E = 256 has one unit with two x tiles and one with one."""
+    cost = {t: dict((x, c) for c, x in units("costs", ONE_SM, 256, t))[nx] for t in (512, T)}
+    cycles = 1965 * (ONE_SM_US[nx][T] - ONE_SM_US[nx][512])
+    assert abs(cost[T] - cost[512] - cycles) < 0.05 * cycles
