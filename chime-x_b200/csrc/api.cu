@@ -46,8 +46,9 @@ void free_plan_device(chx_plan *p) {
 }
 
 // Channel table and work units of the tensor-core kernel for the plan's
-// shape: F channels sharing one TMA map (passed per launch), units of every
-// channel sorted by decreasing cost.
+// shape: F channels sharing one TMA map (passed per launch), and the units of a
+// launch that stores and of one that adds, grouped by CTA: longest first, or, where
+// they are balanced, end to end in channel order.
 cudaError_t build_tc_tables(chx_plan *p) {
     std::vector<ChanDesc> chans(p->F);
     memset(chans.data(), 0, chans.size() * sizeof(ChanDesc));

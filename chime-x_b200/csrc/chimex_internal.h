@@ -96,8 +96,9 @@ struct NvtxRange {
 
 // Launches a kernel that may start its set-up before the stream's previous
 // kernel has ended (programmatic dependent launch).  Such a kernel calls pdl_wait
-// before it touches memory.  Between ordinary launches this GPU spends up to 2 us
-// per kernel boundary.
+// before it touches memory (behind launch_zero: before it touches the output).  Between
+// ordinary launches, which the one-SM tile's kernel and the dp4a kernel keep, this GPU
+// spends up to 2 us per kernel boundary.
 template <class... Params, class... Args>
 cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
                        cudaStream_t st, Args... args) {

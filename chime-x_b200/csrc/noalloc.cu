@@ -47,7 +47,7 @@ constexpr size_t kOffErr = 0;
 constexpr size_t kOffChans = 256;
 constexpr size_t kOffUnits = kOffChans + sizeof(ChanDesc) * kNoAllocMaxChannels;
 constexpr size_t kOffOffsets = kOffUnits + sizeof(Unit) * kNoAllocMaxUnits;
-constexpr size_t kScratchBytes = kOffOffsets + sizeof(int) * (kNoAllocMaxGrid + 1);  // ~162 KiB
+constexpr size_t kScratchBytes = kOffOffsets + sizeof(int) * (kNoAllocMaxGrid + 1);  // ~160 KiB
 static_assert(kOffChans % alignof(ChanDesc) == 0 && kOffUnits % 16 == 0, "table alignment");
 
 // The scratch: error word, channel table, unit table, per-CTA unit offsets.

@@ -308,9 +308,9 @@ __device__ __forceinline__ void xconv(uint32_t w, uint32_t &xr, uint32_t &xi) {
     }
 }
 
-// The SM-pair kernel's y rows, scaled by 2^a (a = 0 or 3, fixed per launch):
-// R = yr 2^a, I = yi 2^a, N = -yr 2^a (and the offset-domain maps alike);
-// tc_pair_correlator.cu says why.
+// y rows scaled by 2^a: R = yr 2^a, I = yi 2^a, N = -yr 2^a (and the offset-domain
+// maps alike).  a = 0 or 3 per launch in the SM-pair kernel (tc_pair_correlator.cu says
+// why), 2 in the kernel for small channels, whose rows are the x operand too.
 //
 // The conversions are bound by the ALU pipe (logic and shifts, half rate), so
 // adds and the left shift are multiply-adds, which run on the other pipe: 6 ALU

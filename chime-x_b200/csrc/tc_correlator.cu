@@ -26,8 +26,8 @@
 // that consecutive MMAs are independent:
 //   Re += R.X    Im += I.X    Re += I.Y    Im += N.Y
 // Every operand row is stored once (a layout interleaving R and I per
-// 8-sample block needed the I rows twice: 16 KiB of y per stage, measured
-// 3-4 % slower on the SM-pair kernel, whose shared-memory traffic bounds it).
+// 8-sample block needed the I rows twice: 16 KiB of y per stage, 3-4 % slower on
+// the SM-pair kernel of the time, which shared-memory traffic bounded).
 //
 // Roles (576 threads, one persistent CTA per SM; each CTA works through its
 // own contiguous range of the unit table, assigned on the host by cost):
@@ -514,11 +514,12 @@ void append_units(std::vector<Unit> &out, int tile, int chan, int E, int t_begin
 // tiles with a half-empty row and column of units, whose missing tile's work
 // is done in vain; the one-SM kernel wastes none but converts two x tiles per
 // y tile on one SM.  Measured on B200 with the automatic split (T = 16384,
-// F = 8, TOPS, SM pair / one SM): E = 1920 2427 / 2024, 1664 1998 / 1775,
-// 1408 2051 / 1953, 1152 1903 / 1611, 896 1514 / 1473, 640 1418 / 1449,
-// 384 953 / 732, and 2048 2741 / 2133.  The SM pair is the default from two
-// tiles up; a single tile (E <= 128) would leave three quarters of its one
-// pair unit empty, so it goes to the one-SM tile.  Both stay available as a
+// F = 8, TOPS, SM pair / one SM): E = 2048 3558 / 1971, 1920 3200 / 1963,
+// 1664 2968 / 1842, 1408 2913 / 1867, 1152 2753 / 2000, 896 2538 / 1844,
+// 640 2174 / 1571, 384 1410 / 1194, 256 1168 / 900.  The SM pair is the default from
+// two tiles up; a single tile (E <= 128) would leave three quarters of its one
+// pair unit empty, so it goes to the one-SM tile (F = 148, T = 4096, us, SM pair / one
+// SM: E = 128 66.8 / 29.5, E = 32 58.6 / 19.4).  Both stay available as a
 // tile option and to the autotuner.  A launch of the one-SM tile whose channels
 // all fit one 128-element tile runs tc_small_correlator.cu's kernel (tc_launch_tile).
 int tc_default_tile(int E) {

@@ -158,7 +158,7 @@ int chx_blocks_to_full(chx_plan *plan, const int32_t *d_blocks, int32_t *d_full,
  * This entry point computes exactly what chx_correlate computes for a plan
  * of (E, F, T, upper_triangle_convention), needs no plan and calls no
  * allocator: its work tables live in a fixed-size array inside the library
- * (about 162 KiB on every GPU that loads it, kept until exit), written on the
+ * (about 160 KiB on every GPU that loads it, kept until exit), written on the
  * device by a small kernel from its launch parameters.  It uses the plan
  * path's default tile variant and cuts sample ranges only where int32
  * exactness requires it (no automatic split).  Limits: F <= 64 channels and
